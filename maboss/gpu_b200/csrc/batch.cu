@@ -25,13 +25,20 @@ namespace mb {
 
 namespace {
 
-// compaction of one variant's fixed-point table into (state, count) records
-__global__ void mbb_fixed_extract(unsigned cap, int words, const mb_key128* __restrict__ keys,
+// compaction of one variant's fixed-point table into (state, count) records; the first `tail_blocks`
+// blocks add the window sums of the trajectories that mb_record_fixed counted
+__global__ void __launch_bounds__(32 * MB_TAIL_COLS) mbb_fixed_extract(mb_stats_params p, float max_time,
+								  unsigned tail_blocks, unsigned cap, int words, const mb_key128* __restrict__ keys,
 								  const unsigned* __restrict__ counts, const unsigned* __restrict__ states,
 								  unsigned* __restrict__ out_n, unsigned* __restrict__ out_states,
 								  unsigned* __restrict__ out_counts)
 {
-	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (blockIdx.x < tail_blocks)
+	{
+		mb_tail_add(p, max_time, blockIdx.x * MB_TAIL_COLS);
+		return;
+	}
+	const unsigned i = (blockIdx.x - tail_blocks) * blockDim.x + threadIdx.x;
 	if (i >= cap)
 		return;
 	const mb_key128 k = keys[i];
@@ -493,7 +500,7 @@ void batch_engine::enqueue(prepared& ps, cudaStream_t s, bool capturing)
 	{
 		variant& V = *vars_[i];
 		const host_off_t& o = ps.host_off[i];
-		V.st.extract(s, V.out_states.as<unsigned>(), V.out_counts.as<unsigned>());
+		V.st.extract(s, V.out_states.as<unsigned>(), V.out_counts.as<unsigned>(), print6(nets[V.net]->L.max_time));
 		dbuf& win = V.st.occ.bytes > 8 ? V.st.occ : V.st.cnt;
 		MB_CUDA(cudaMemcpyAsync(host + o.win, win.p, win.bytes, cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaMemcpyAsync(host + o.h, V.st.h.p, V.st.h.bytes, cudaMemcpyDeviceToHost, s));
@@ -650,6 +657,11 @@ void plain_stats::init_plain(int words, float tick, float tmax, bool discrete, c
 	fx_h = std::ldexp(1.0, entropy_exponent(n, tick, discrete));
 	const size_t cells = (size_t)n_windows * n_bins;
 	occ.alloc(discrete ? 8 : cells * sizeof(long long));
+	if (!discrete && cells <= tail_max_cells)
+	{
+		tail.alloc(cells * sizeof(unsigned));
+		MB_CUDA(cudaMemsetAsync(tail.p, 0, tail.bytes, s)); // (each run leaves it cleared)
+	}
 	cnt.alloc(discrete ? cells * sizeof(unsigned) : 4);
 	h.alloc(n_windows * sizeof(long long));
 	fin.alloc(n_bins * sizeof(unsigned));
@@ -678,6 +690,7 @@ void plain_stats::init_plain(int words, float tick, float tmax, bool discrete, c
 	p.fp_states = fp_states.as<unsigned>();
 	p.fp_mask = cap - 1;
 	p.fp_overflow = counters.as<unsigned>();
+	p.tail = tail.as<unsigned>();
 }
 
 void plain_stats::zero(cudaStream_t s)
@@ -686,11 +699,13 @@ void plain_stats::zero(cudaStream_t s)
 		MB_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, s));
 }
 
-void plain_stats::extract(cudaStream_t s, unsigned* out_states, unsigned* out_counts)
+void plain_stats::extract(cudaStream_t s, unsigned* out_states, unsigned* out_counts, float sim_max_time)
 {
 	unsigned* out_n = counters.as<unsigned>() + 1;
-	mbb_fixed_extract<<<(fp_cap + 255) / 256, 256, 0, s>>>(fp_cap, W, p.fp_keys, p.fp_counts, p.fp_states, out_n,
-														  out_states, out_counts);
+	const unsigned tail_blocks = p.tail ? (n_bins + MB_TAIL_COLS - 1) / MB_TAIL_COLS : 0u;
+	constexpr unsigned threads = 32 * MB_TAIL_COLS;
+	mbb_fixed_extract<<<tail_blocks + (fp_cap + threads - 1) / threads, threads, 0, s>>>(
+		p, sim_max_time, tail_blocks, fp_cap, W, p.fp_keys, p.fp_counts, p.fp_states, out_n, out_states, out_counts);
 	MB_CUDA(cudaGetLastError());
 }
 

@@ -19,7 +19,7 @@ namespace mb {
 // compiled module).
 struct plain_stats
 {
-	dbuf occ, cnt, h, fin, fp_keys, fp_counts, fp_states, counters;
+	dbuf occ, cnt, h, fin, fp_keys, fp_counts, fp_states, counters, tail;
 	unsigned fp_cap = 0;
 	int W = 1, n_windows = 0;
 	unsigned n_bins = 0;
@@ -32,7 +32,9 @@ struct plain_stats
 					cudaStream_t s);
 	void zero(cudaStream_t s); // clear every accumulator (asynchronous, capturable)
 	// compact the fixed-point table into (state, count) records; their number goes to counters[1]
-	void extract(cudaStream_t s, unsigned* out_states, unsigned* out_counts);
+	// (and add the window sums of the trajectories counted at their fixed point; `sim_max_time` is the
+	// generated code's max_time)
+	void extract(cudaStream_t s, unsigned* out_states, unsigned* out_counts, float sim_max_time);
 	// the result from host copies of the accumulators and the device records of the fixed points
 	std::unique_ptr<result> result_from(const void* win, const void* h, const void* fin, const void* counters,
 										const unsigned* out_states, const unsigned* out_counts, long long n,

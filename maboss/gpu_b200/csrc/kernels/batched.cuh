@@ -292,8 +292,8 @@ __device__ __forceinline__ void mbb_grad_slice(const mb_variant& var, const mbb_
 
 template <bool GRAD>
 __device__ __forceinline__ void mbb_record(const mb_variant& var, const mbb_lane& v, int P, mb_win_acc& acc,
-										   unsigned idx, float t0, float t1, float h, bool discrete, float tick,
-										   double& C1, double& C2, mbb_cot_cache& cc)
+										   unsigned idx, float t0, float t1, float h, bool fixed, bool discrete,
+										   float tick, double& C1, double& C2, mbb_cot_cache& cc)
 {
 	if (t1 == 0.f)
 		return;
@@ -308,7 +308,10 @@ __device__ __forceinline__ void mbb_record(const mb_variant& var, const mbb_lane
 		}
 		return;
 	}
-	mb_record_cont(acc, var.st, var.st.win_h, idx, t0, t1, h);
+	if (fixed)
+		mb_record_fixed(acc, var.st, var.st.win_h, idx, t0, t1);
+	else
+		mb_record_cont(acc, var.st, var.st.win_h, idx, t0, t1, h);
 	if (GRAD)
 	{
 		// the same window slices as mb_record_cont
@@ -503,39 +506,43 @@ __device__ void mbb_body(const mb_batch_params& B)
 			const NET net(B, var);
 			const bool discrete = net.discrete();
 			const float max_time = net.max_time(), tick = net.tick();
+			if (total == 0)
+			{
+				// a fixed point: the state stays until max_time
+				running = false;
+				mbb_record<GRAD>(var, v, P, acc, idx, time, max_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
+				atomicAdd(var.st.final_cnt + idx, 1u);
+				unsigned st[64];
+				const int W = net.W() < 64 ? net.W() : 64;
+				for (int w = 0; w < W; w++)
+					st[w] = v.S(w);
+				mb_fixed_insert_rt(var.st, st, W);
+				if (GRAD)
+					mbb_grad_end(v, P, discrete, C1, C2);
+				atomicAdd(var.transitions, trans + 1);
+				trans = 0;
+				break;
+			}
 			const uint4 rb = curand4(&rng);
 			float tn;
-			if (total == 0)
-				tn = max_time;
+			if (discrete)
+			{
+				tn = time + tick;
+				tn = max_time - tick < tn ? max_time : tn;
+			}
 			else
 			{
-				if (discrete)
-				{
-					tn = time + tick;
-					tn = max_time - tick < tn ? max_time : tn;
-				}
-				else
-				{
-					const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
-					tn = time + -logf(u) / ((float)total * (1.0f / (float)(1u << var.rate_shift)));
-				}
-				tn = fminf(tn, max_time);
+				const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
+				tn = time + -logf(u) / ((float)total * (1.0f / (float)(1u << var.rate_shift)));
 			}
+			tn = fminf(tn, max_time);
 			trans += (tn != 0.f) ? 1ull : 0ull;
-			mbb_record<GRAD>(var, v, P, acc, idx, time, tn, total == 0 ? 0.f : h, discrete, var.st.win_tick, C1, C2, cc);
+			mbb_record<GRAD>(var, v, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
 			time = tn;
 			if (time >= max_time)
 			{
 				running = false;
 				atomicAdd(var.st.final_cnt + idx, 1u);
-				if (total == 0)
-				{
-					unsigned st[64];
-					const int W = net.W() < 64 ? net.W() : 64;
-					for (int w = 0; w < W; w++)
-						st[w] = v.S(w);
-					mb_fixed_insert_rt(var.st, st, W);
-				}
 				if (GRAD)
 					mbb_grad_end(v, P, discrete, C1, C2);
 				atomicAdd(var.transitions, trans);

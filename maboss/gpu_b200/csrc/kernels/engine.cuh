@@ -78,13 +78,10 @@ __device__ void mb_fixed_insert(const mb_stats_params& p, const state_word_t* st
 {
 	const mb_key128 key = mb_state_key(st);
 	const unsigned h = (unsigned)mb_mix64(key.lo ^ mb_mix64(key.hi));
-	mb_key128 empty;
-	empty.lo = 0;
-	empty.hi = 0;
 	for (unsigned probe = 0; probe <= p.fp_mask; probe++)
 	{
 		const unsigned slot = (h + probe) & p.fp_mask;
-		const mb_key128 prev = atomicCAS(p.fp_keys + slot, empty, key);
+		const mb_key128 prev = mb_fixed_claim(p.fp_keys + slot, key);
 		if (prev.lo == 0ull && prev.hi == 0ull)
 		{
 #pragma unroll
@@ -110,6 +107,8 @@ __device__ __forceinline__ void mb_record(mb_win_acc& a, const mb_stats_params& 
 	const mb_idx_t idx = get_non_internal_index(st);
 	if (discrete_time)
 		mb_record_disc(p, hsink, idx, t0, h);
+	else if (t1 == max_time && h == 0.f) // at a fixed point, or as good as one for the window sums
+		mb_record_fixed(a, p, hsink, idx, t0, t1);
 	else
 		mb_record_cont(a, p, hsink, idx, t0, t1, h);
 }
@@ -667,10 +666,7 @@ extern "C" __global__ void __launch_bounds__(128) mb_fused_exact(mb_fused_params
 		// (+1.6 % on the 1000-node network; as in the fast kernel)
 		for (int step = 0; step < MB_STEPS_PER_PASS && running; step++)
 		{
-		float total = 0.f, h = 0.f, tn = 0.f;
-		if (running)
-		{
-			total = mb_exact_total(v, lo);
+			const float total = mb_exact_total(v, lo);
 			lo = state_words;
 			if (isinf(total))
 			{
@@ -678,54 +674,55 @@ extern "C" __global__ void __launch_bounds__(128) mb_fused_exact(mb_fused_params
 				atomicAdd(P.errors, 1u);
 				running = false;
 				mb_final_add(P.st, idx);
+				break;
 			}
-			else if (total == 0.f)
-				tn = max_time;
-			else
+			if (total == 0.f)
 			{
+				// a fixed point: the state stays until max_time
+				running = false;
+				trans++;
 				if (discrete_time)
-				{
-					tn = time + time_tick;
-					tn = max_time - time_tick < tn ? max_time : tn;
-				}
+					mb_record_disc(P.st, hsink, idx, time, 0.f);
 				else
-					tn = time + -logf(curand_uniform(&rng)) / total;
-				tn = fminf(tn, max_time);
-				if (h_stale)
-					h_cache = mb_exact_entropy(v);
-				h_stale = false;
-				h = h_cache;
+					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				mb_final_add(P.st, idx);
+				state_word_t st[state_words];
+#pragma unroll
+				for (int w = 0; w < state_words; w++)
+					st[w] = v.S(w);
+				mb_fixed_insert(P.st, st);
+				break;
 			}
-		}
-		if (running)
-		{
+			float tn;
+			if (discrete_time)
+			{
+				tn = time + time_tick;
+				tn = max_time - time_tick < tn ? max_time : tn;
+			}
+			else
+				tn = time + -logf(curand_uniform(&rng)) / total;
+			tn = fminf(tn, max_time);
+			if (h_stale)
+				h_cache = mb_exact_entropy(v);
+			h_stale = false;
 			trans += (tn != 0.f) ? 1ull : 0ull;
 			if (tn != 0.f)
 			{
 				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, h);
+					mb_record_disc(P.st, hsink, idx, time, h_cache);
 				else
-					mb_record_cont(acc, P.st, hsink, idx, time, tn, h);
+					mb_record_cont(acc, P.st, hsink, idx, time, tn, h_cache);
 			}
 			time = tn;
 			if (time >= max_time)
 			{
 				running = false;
 				mb_final_add(P.st, idx);
-				if (total == 0.f)
-				{
-					state_word_t st[state_words];
-#pragma unroll
-					for (int w = 0; w < state_words; w++)
-						st[w] = v.S(w);
-					mb_fixed_insert(P.st, st);
-				}
 			}
 			else if (P.traj_len > 1 && ++slot >= P.traj_len)
 				slot = 1; // epoch boundary: the next epoch re-evaluates the same state
 			else
 				lo = mb_exact_flip(v, mb_exact_select(v, curand_uniform(&rng) * total), idx, h_stale);
-		}
 		}
 		__syncwarp();
 	}
@@ -839,47 +836,50 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 		// 50-node one; a lane whose trajectory ends idles for the rest of the pass)
 		for (int step = 0; step < MB_STEPS_PER_PASS && running; step++)
 		{
+			if (total == 0)
+			{
+				// a fixed point: the state stays until max_time
+				running = false;
+				trans++;
+				if (discrete_time)
+					mb_record_disc(P.st, hsink, idx, time, 0.f);
+				else
+					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				mb_final_add(P.st, idx);
+				state_word_t st[state_words];
+#pragma unroll
+				for (int w = 0; w < state_words; w++)
+					st[w] = v.S(w);
+				mb_fixed_insert(P.st, st);
+				break;
+			}
 			const uint4 rb = curand4(&rng); // x: waiting time, (y, z): flip
 			float tn;
-			if (total == 0)
-				tn = max_time;
+			if (discrete_time)
+			{
+				tn = time + time_tick;
+				tn = max_time - time_tick < tn ? max_time : tn;
+			}
 			else
 			{
-				if (discrete_time)
-				{
-					tn = time + time_tick;
-					tn = max_time - time_tick < tn ? max_time : tn;
-				}
-				else
-				{
-					// uniform in (0, 1]: the top 24 bits plus one, times 2^-24
-					const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
-					tn = time + -logf(u) / ((float)total * inv_scale);
-				}
-				tn = fminf(tn, max_time);
+				// uniform in (0, 1]: the top 24 bits plus one, times 2^-24
+				const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
+				tn = time + -logf(u) / ((float)total * inv_scale);
 			}
+			tn = fminf(tn, max_time);
 			trans += (tn != 0.f) ? 1ull : 0ull;
 			if (tn != 0.f)
 			{
 				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, total == 0 ? 0.f : h);
+					mb_record_disc(P.st, hsink, idx, time, h);
 				else
-					mb_record_cont(acc, P.st, hsink, idx, time, tn, total == 0 ? 0.f : h);
+					mb_record_cont(acc, P.st, hsink, idx, time, tn, h);
 			}
 			time = tn;
 			if (time >= max_time)
 			{
-				// end of the trajectory: final state, fixed point
 				running = false;
 				mb_final_add(P.st, idx);
-				if (total == 0)
-				{
-					state_word_t st[state_words];
-#pragma unroll
-					for (int w = 0; w < state_words; w++)
-						st[w] = v.S(w);
-					mb_fixed_insert(P.st, st);
-				}
 			}
 			else
 			{
@@ -1449,13 +1449,22 @@ extern "C" __global__ void __launch_bounds__(MB_SCAN_BLOCK)
 }
 
 
-// ---- compaction of the fixed-point table into (state, count) records
-extern "C" __global__ void mb_fixed_extract(unsigned cap, const mb_key128* __restrict__ keys,
-											 const unsigned* __restrict__ counts, const uint32_t* __restrict__ states,
-											 unsigned* __restrict__ out_n, uint32_t* __restrict__ out_states,
-											 unsigned* __restrict__ out_counts)
+// ---- compaction of the fixed-point table into (state, count) records; the first `tail_blocks` blocks
+// add the window sums of the trajectories that mb_record_fixed counted (dense histograms; in this
+// launch because a small run is as long as its launches)
+extern "C" __global__ void __launch_bounds__(32 * MB_TAIL_COLS)
+	mb_fixed_extract(mb_stats_params p, unsigned tail_blocks, unsigned cap, const mb_key128* __restrict__ keys,
+					 const unsigned* __restrict__ counts, const uint32_t* __restrict__ states,
+					 unsigned* __restrict__ out_n, uint32_t* __restrict__ out_states, unsigned* __restrict__ out_counts)
 {
-	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (blockIdx.x < tail_blocks)
+	{
+#ifndef MBG_WIDE_INDEX
+		mb_tail_add(p, max_time, blockIdx.x * MB_TAIL_COLS);
+#endif
+		return;
+	}
+	const unsigned i = (blockIdx.x - tail_blocks) * blockDim.x + threadIdx.x;
 	if (i >= cap)
 		return;
 	const mb_key128 k = keys[i];

@@ -31,7 +31,14 @@ struct mb_stats_params
 	long long* bin_vals;  // [cap]
 	unsigned bin_mask;	  // cap - 1
 	unsigned* bin_overflow;
+	// [T*S] trajectories at a fixed point from window w on, per non-internal state (continuous time,
+	// dense histograms of at most tail_max_cells); mb_tail_add turns them into window sums. Null: every
+	// window of such a trajectory is added on its own
+	unsigned* tail;
 };
+
+// One block's warps take this many neighbouring histogram columns in mb_tail_add.
+constexpr int MB_TAIL_COLS = 8;
 
 struct mb_fused_params
 {

@@ -501,7 +501,9 @@ void stats_state::init(module& m, float tick, float tmax, bool discrete, const s
 		}
 		else
 		{
-			occ.alloc(cells * sizeof(long long));
+			// the counts of trajectories at a fixed point behind the sums: one clear for both
+			has_tail = cells <= tail_max_cells;
+			occ.alloc(cells * (sizeof(long long) + (has_tail ? sizeof(unsigned) : 0)));
 			MB_CUDA(cudaMemsetAsync(occ.p, 0, occ.bytes, s));
 		}
 		h.alloc(n_windows * sizeof(long long));
@@ -547,6 +549,7 @@ void stats_state::init(module& m, float tick, float tmax, bool discrete, const s
 	p.bin_mask = bin_cap ? bin_cap - 1 : 0;
 	p.fp_overflow = fp_overflow_ctr();
 	p.bin_overflow = bin_overflow_ctr();
+	p.tail = has_tail ? reinterpret_cast<unsigned*>(occ.as<long long>() + cells) : nullptr;
 }
 
 void stats_state::zero(cudaStream_t s)
@@ -620,6 +623,29 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 	r.sections = sections;
 	r.wide = wide;
 	const size_t cells = (size_t)n_windows * n_bins;
+	// compact the occupied fixed-point slots on the device; the same launch adds the window sums of the
+	// trajectories that were counted at their fixed point (and clears the counts)
+	MB_CUDA(cudaMemsetAsync(extract_ctr(), 0, sizeof(unsigned), s));
+	// compaction buffers, allocated with the first result and kept for the next runs
+	if (fp_cap && out_counts.bytes != (size_t)fp_cap * sizeof(unsigned))
+	{
+		out_counts.alloc((size_t)fp_cap * sizeof(unsigned));
+		out_states.alloc((size_t)fp_cap * m.state_words * sizeof(unsigned));
+	}
+	if (fp_cap || p.tail)
+	{
+		unsigned cap = fp_cap, tail_blocks = p.tail ? (n_bins + MB_TAIL_COLS - 1) / MB_TAIL_COLS : 0u;
+		mb_stats_params sp = p;
+		mb_key128* keys = p.fp_keys;
+		unsigned* counts = p.fp_counts;
+		unsigned* states = p.fp_states;
+		unsigned* out_n = extract_ctr();
+		unsigned* os = out_states.as<unsigned>();
+		unsigned* oc = out_counts.as<unsigned>();
+		void* args[] = { &sp, &tail_blocks, &cap, &keys, &counts, &states, &out_n, &os, &oc };
+		constexpr unsigned threads = 32 * MB_TAIL_COLS;
+		mb::launch(m.fixed_extract, tail_blocks + (cap + threads - 1) / threads, threads, 0, s, args);
+	}
 	if (wide)
 	{
 		// compact the occupied bins on the device, then sort them (and merge any key that two
@@ -737,27 +763,7 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 		MB_CUDA(cudaMemcpyAsync(r.final_cnt.data(), fin.p, n_bins * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
 	}
 
-	// count occupied fixed-point slots, then compact them on the device and copy the records
 	unsigned ctr[8];
-	MB_CUDA(cudaMemsetAsync(extract_ctr(), 0, sizeof(unsigned), s));
-	// compaction buffers, allocated with the first result and kept for the next runs
-	if (fp_cap && out_counts.bytes != (size_t)fp_cap * sizeof(unsigned))
-	{
-		out_counts.alloc((size_t)fp_cap * sizeof(unsigned));
-		out_states.alloc((size_t)fp_cap * m.state_words * sizeof(unsigned));
-	}
-	if (fp_cap)
-	{
-		unsigned cap = fp_cap;
-		mb_key128* keys = p.fp_keys;
-		unsigned* counts = p.fp_counts;
-		unsigned* states = p.fp_states;
-		unsigned* out_n = extract_ctr();
-		unsigned* os = out_states.as<unsigned>();
-		unsigned* oc = out_counts.as<unsigned>();
-		void* args[] = { &cap, &keys, &counts, &states, &out_n, &os, &oc };
-		launch(m.fixed_extract, (cap + 255) / 256, 256, 0, s, args);
-	}
 	unsigned long long trans = 0;
 	MB_CUDA(cudaMemcpyAsync(ctr, counters.p, sizeof ctr, cudaMemcpyDeviceToHost, s));
 	MB_CUDA(cudaMemcpyAsync(&trans, transitions(), sizeof trans, cudaMemcpyDeviceToHost, s));

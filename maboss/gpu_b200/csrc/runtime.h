@@ -189,6 +189,11 @@ run_config config_from_layout(const model_layout& L, int mode);
 // their non-zero cells only, when those are at most a quarter of the cells.
 constexpr unsigned long long compact_min_cells = 1ull << 24;
 
+// Dense continuous histograms of at most this many cells keep a count of the trajectories at a fixed
+// point beside each cell (mb_record_fixed): 16 MB at most, cleared and scanned once a run in 20 us. Above
+// it each window of such a trajectory is added on its own, and no second large array is kept.
+constexpr unsigned long long tail_max_cells = 1ull << 22;
+
 struct result
 {
 	int state_size = 0, state_words = 0, n_windows = 0;
@@ -266,6 +271,7 @@ struct stats_state
 	std::unique_ptr<long long[], host_deleter> hbin_vals;
 	size_t hbin_cap = 0;
 	bool wide = false;
+	bool has_tail = false; // occ is followed by the counts of mb_record_fixed (u32 per cell)
 	unsigned fp_cap = 0;
 	int n_windows = 0;
 	unsigned n_bins = 0;
