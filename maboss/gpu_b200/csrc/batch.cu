@@ -77,7 +77,7 @@ int batch_engine::add_model(const model_t& m)
 	net->model = m;
 	net->L = analyze_model(m);
 	const model_layout& L = net->L;
-	if (!L.all_fast_path || !L.incremental_ok)
+	if (!L.all_fast_path || !L.incremental_ok || L.max_inputs > incremental_record_inputs)
 		throw engine_error(MB_ERR_INVALID, "batched runs need every rate in the form rate_up = @logic ? U : 0; "
 										   "rate_down = @logic ? 0 : D with at most 12 logic inputs per node");
 	if (L.state_words > 64)

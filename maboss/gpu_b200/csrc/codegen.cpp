@@ -185,6 +185,55 @@ void collect_nodes(const model_t& m, const expr& e, const std::string& current, 
 	}
 }
 
+// The truth table of a logic made of nodes, aliases, the literals 0 and 1, NOT, AND, OR and XOR alone, 32
+// input patterns at a time (pattern p has input `in[t]` at bit t of p). False for other logics, which
+// eval_c evaluates pattern by pattern: 33 ms instead of 1 for the 133-node example model.
+bool eval_bits(const model_t& m, const expr& e, const std::string& current, const std::vector<int>& in,
+			   std::vector<unsigned>& out)
+{
+	using K = expr::kind_t;
+	static const unsigned low[5] = { 0xaaaaaaaau, 0xccccccccu, 0xf0f0f0f0u, 0xff00ff00u, 0xffff0000u };
+	switch (e.kind)
+	{
+		case K::literal:
+			if (e.value != 0.f && e.value != 1.f)
+				return false;
+			std::fill(out.begin(), out.end(), e.value != 0.f ? ~0u : 0u);
+			return true;
+		case K::identifier:
+		{
+			const auto it = std::find(in.begin(), in.end(), m.node_index(e.name));
+			if (it == in.end())
+				return false;
+			const int t = (int)(it - in.begin());
+			for (size_t w = 0; w < out.size(); w++)
+				out[w] = t < 5 ? low[t] : ((w >> (t - 5)) & 1) ? ~0u : 0u;
+			return true;
+		}
+		case K::alias:
+			return eval_bits(m, m.nodes[m.node_index(current)].get_attr(e.name.substr(1)), current, in, out);
+		case K::paren: return eval_bits(m, *e.a, current, in, out);
+		case K::unary:
+			if (e.op != op_t::NOT || !eval_bits(m, *e.a, current, in, out))
+				return false;
+			for (unsigned& x : out)
+				x = ~x;
+			return true;
+		case K::binary:
+		{
+			if (e.op != op_t::AND && e.op != op_t::OR && e.op != op_t::XOR)
+				return false;
+			std::vector<unsigned> b(out.size());
+			if (!eval_bits(m, *e.a, current, in, out) || !eval_bits(m, *e.b, current, in, b))
+				return false;
+			for (size_t w = 0; w < out.size(); w++)
+				out[w] = e.op == op_t::AND ? out[w] & b[w] : e.op == op_t::OR ? out[w] | b[w] : out[w] ^ b[w];
+			return true;
+		}
+		default: return false;
+	}
+}
+
 // generator.cpp:57-82 (is_logic_ternary_expression). The reference evaluates the branches
 // unconditionally and aborts on non-constant ones; here such nodes use the general form.
 bool is_logic_ternary(const model_t& m, const expr* e, bool up, float& val)
@@ -240,6 +289,12 @@ void emit_array(std::ostream& os, const char* type, const char* name, const std:
 //   crec[r]    = {k | m << 16 | (ni_pos(k) + 1) << 21, truth table or offset, inputs 0-1, inputs 2-3}
 // with inputs 4..11 in cext[r], read only for logics of more than 4 inputs. The truth table of k is
 // inline when it has at most 5 inputs (32 patterns), else an offset into tt.
+// A model with logics of 13 to 16 inputs defines MBG_INCREMENTAL_MANY instead: its exact and epoch
+// kernels are incremental (inputs 12-15 in mbg_inc_cext2), fast mode keeps the dense kernel, whose
+// trajectories differ from the incremental one's. The 133-node example model has two nodes of 13
+// inputs; its dense exact kernel needs 254 registers and evaluates 133 rate functions per step:
+// 1e6 trajectories
+// 110 ms dense, 61 ms incremental.
 void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 {
 	ss << std::endl << "// ---- incremental engine tables" << std::endl;
@@ -256,7 +311,8 @@ void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 						  std::to_string(v[i + 2]) + "u, " + std::to_string(v[i + 3]) + "u}");
 		return out;
 	};
-	ss << "#define MBG_INCREMENTAL 1" << std::endl;
+	const bool many = L.max_inputs > incremental_record_inputs;
+	ss << (many ? "#define MBG_INCREMENTAL_MANY 1" : "#define MBG_INCREMENTAL 1") << std::endl;
 	// the fast kernel's integer rates (else fast mode takes the dense fp32 kernel)
 	if (t.ok && L.integer_rates_ok)
 		ss << "#define MBG_INTEGER_RATES 1" << std::endl;
@@ -281,6 +337,13 @@ void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 	// 16-byte dependent records (the node's rates come from mbg_inc_q); inputs 4-11 apart
 	emit_array(ss, "uint4", "mbg_inc_crec", u4(t.crec));
 	emit_array(ss, "uint4", "mbg_inc_cext", u4(t.cext));
+	if (many)
+	{
+		std::vector<std::string> e2;
+		for (size_t i = 0; i + 1 < t.cext2.size(); i += 2)
+			e2.push_back("{" + std::to_string(t.cext2[i]) + "u, " + std::to_string(t.cext2[i + 1]) + "u}");
+		emit_array(ss, "uint2", "mbg_inc_cext2", e2);
+	}
 	emit_array(ss, "unsigned", "mbg_inc_tt", t.tt);
 	emit_array(ss, "int", "mbg_inc_self", t.self);
 	// float rates (up, down) of every node as the generated rate functions return them (exact mode)
@@ -480,14 +543,21 @@ model_layout analyze_model(const model_t& m)
 	// words (19200 nodes) fit a block of 32 threads; larger models take the dense kernels
 	// (the incremental exact kernel's binary search over word-end rate sums needs rates >= 0)
 	L.incremental_ok = L.all_fast_path && L.rates_nonnegative && N <= 65535 && L.state_words <= 600;
-	constexpr int max_inputs = 12;
+	// a logic of 13 to 16 inputs has 2^13 to 2^16 patterns: at most 2^18 of them in a model (32 KB of
+	// tables, and at worst 0.5 s where eval_c has to evaluate them), else the dense kernels
+	constexpr int max_inputs = 16;
+	long long wide_patterns = 0;
 	if (L.incremental_ok)
 	{
 		std::vector<std::set<int>> inputs(N);
 		for (int i = 0; i < N && L.incremental_ok; i++)
 		{
 			collect_nodes(m, m.nodes[i].get_attr("logic"), m.nodes[i].name, inputs[i]);
-			if ((int)inputs[i].size() > max_inputs)
+			const int mi = (int)inputs[i].size();
+			L.max_inputs = std::max(L.max_inputs, mi);
+			if (mi > incremental_record_inputs && mi <= max_inputs)
+				wide_patterns += 1LL << mi;
+			if (mi > max_inputs || wide_patterns > (1LL << 18))
 				L.incremental_ok = false;
 		}
 		if (L.incremental_ok)
@@ -511,15 +581,21 @@ model_layout analyze_model(const model_t& m)
 				const int patterns = 1 << mi;
 				const int words = (patterns + 31) / 32;
 				std::vector<unsigned> tt(words, 0u);
+				const expr& logic = m.nodes[i].get_attr("logic");
+				const bool bits = eval_bits(m, logic, m.nodes[i].name, in, tt);
+				if (patterns < 32)
+					tt[0] &= (1u << patterns) - 1u;
+				if (!bits)
+					std::fill(tt.begin(), tt.end(), 0u);
 				try
 				{
-					for (int p = 0; p < patterns; p++)
+					for (int p = 0; p < patterns && !bits; p++)
 					{
 						auto bit = [&](int node) {
 							auto it = std::find(in.begin(), in.end(), node);
 							return ((p >> (it - in.begin())) & 1) != 0;
 						};
-						cval v = eval_c(m, m.nodes[i].get_attr("logic"), m.nodes[i].name, bit);
+						cval v = eval_c(m, logic, m.nodes[i].name, bit);
 						if (v.truthy())
 							tt[p / 32] |= 1u << (p % 32);
 					}
@@ -545,7 +621,7 @@ model_layout analyze_model(const model_t& m)
 			L.rate_shift = integer_rate_shift(L.up, L.down, L.state_words);
 			L.q_up.resize(N);
 			L.q_down.resize(N);
-			L.integer_rates_ok = true;
+			L.integer_rates_ok = L.max_inputs <= incremental_record_inputs;
 			for (int i = 0; i < N; i++)
 			{
 				for (int which = 0; which < 2; which++)
@@ -658,6 +734,7 @@ incremental_tables build_incremental_tables(const model_layout& L, const std::ve
 	for (size_t k = 0; k < L.noninternal_nodes.size(); k++)
 		ni_pos[L.noninternal_nodes[k]] = (int)k;
 	t.self.assign(N, -1);
+	std::vector<int> tt_at(N, -1); // a node's truth table is stored once, for all records of the node
 	auto push4 = [](std::vector<unsigned>& v, unsigned a, unsigned b, unsigned c, unsigned d) {
 		v.push_back(a);
 		v.push_back(b);
@@ -680,8 +757,12 @@ incremental_tables build_incremental_tables(const model_layout& L, const std::ve
 				ttw = L.tt_words[t0];
 			else
 			{
-				ttw = (unsigned)t.tt.size();
-				t.tt.insert(t.tt.end(), L.tt_words.begin() + t0, L.tt_words.begin() + t0 + nt);
+				if (tt_at[k] < 0)
+				{
+					tt_at[k] = (int)t.tt.size();
+					t.tt.insert(t.tt.end(), L.tt_words.begin() + t0, L.tt_words.begin() + t0 + nt);
+				}
+				ttw = (unsigned)tt_at[k];
 			}
 			push4(t.hdr, (unsigned)k | ((unsigned)m << 16) | ((unsigned)(ni_pos[k] + 1) << 21), qu[k], qd[k], ttw);
 			unsigned in[16] = { 0 };
@@ -692,6 +773,8 @@ incremental_tables build_incremental_tables(const model_layout& L, const std::ve
 			push4(t.crec, (unsigned)k | ((unsigned)m << 16) | ((unsigned)(ni_pos[k] + 1) << 21), ttw,
 				  in[0] | in[1] << 16, in[2] | in[3] << 16);
 			push4(t.cext, in[4] | in[5] << 16, in[6] | in[7] << 16, in[8] | in[9] << 16, in[10] | in[11] << 16);
+			t.cext2.push_back(in[12] | in[13] << 16);
+			t.cext2.push_back(in[14] | in[15] << 16);
 		}
 	}
 	if (t.tt.empty())

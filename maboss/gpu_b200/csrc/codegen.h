@@ -40,6 +40,7 @@ struct model_layout
 	// Incremental engine tables (valid when `incremental_ok`): node -> inputs of its logic
 	// (CSR), the logic truth table over those inputs, and node -> dependents (CSR).
 	bool incremental_ok = false;
+	int max_inputs = 0; // the most inputs of a node's logic (valid when `incremental_ok`)
 	std::vector<int> in_ptr, in_idx;
 	std::vector<int> tt_ptr;				// offset (in 32-bit words) of each node's truth table
 	std::vector<unsigned> tt_words;			// truth tables, bit b = logic value for input pattern b
@@ -79,6 +80,7 @@ struct incremental_tables
 	// compact dependent records (the NVRTC kernels): {k | m << 16 | (ni_pos(k) + 1) << 21, truth
 	// table or offset, inputs 0-1, inputs 2-3}, and inputs 4-11 of records with more than 4 inputs
 	std::vector<unsigned> crec, cext;
+	std::vector<unsigned> cext2; // two words: inputs 12-15 (models with such logics only)
 	std::vector<unsigned> tt;
 	std::vector<int> self;
 	std::vector<unsigned> q; // (q_up, q_down) per node
@@ -91,6 +93,9 @@ constexpr double integer_rate_min_units = 1048576.0;
 
 incremental_tables build_incremental_tables(const model_layout& L, const std::vector<float>& up,
 											const std::vector<float>& down);
+
+// Logics of more inputs than this take a second extension record (exact and epoch modes only).
+constexpr int incremental_record_inputs = 12;
 
 // The generated CUDA source for a model (model-specific part only).
 std::string generate_code(const model_t& m);

@@ -13,6 +13,11 @@
 // every sum independent of thread order, so results are reproducible bit for bit.
 #include <curand_kernel.h>
 
+// logics of 13 to 16 inputs: incremental exact and epoch kernels, dense fast kernel
+#ifdef MBG_INCREMENTAL_MANY
+#define MBG_INCREMENTAL 1
+#endif
+
 enum class trajectory_status : uint8_t
 {
 	CONTINUE,
@@ -301,6 +306,22 @@ __device__ __forceinline__ bool mb_incr_logic(const mb_incr_view& v, int r, cons
 				p |= ((v.S(node >> 5) >> (node & 31)) & 1u) << t;
 			}
 		}
+#ifdef MBG_INCREMENTAL_MANY
+		if (m > 12)
+		{
+			const uint2 ext2 = __ldg(mbg_inc_cext2 + r);
+			const unsigned ins3[2] = { ext2.x, ext2.y };
+#pragma unroll
+			for (int t = 12; t < 16; t++)
+			{
+				if (t < m)
+				{
+					const unsigned node = (ins3[(t - 12) >> 1] >> ((t & 1) * 16)) & 0xffffu;
+					p |= ((v.S(node >> 5) >> (node & 31)) & 1u) << t;
+				}
+			}
+		}
+#endif
 	}
 	const unsigned ttw = m <= 5 ? rec.y : __ldg(mbg_inc_tt + rec.y + (p >> 5));
 	return (ttw >> (p & 31)) & 1u;

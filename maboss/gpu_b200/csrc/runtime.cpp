@@ -268,7 +268,8 @@ std::unique_ptr<module> compile_module(context& ctx, const std::string& generate
 	m->state_size = parse_constexpr(generated_code, "state_size", -1);
 	m->state_words = parse_constexpr(generated_code, "state_words", -1);
 	m->noninternal_count = parse_constexpr(generated_code, "mbg_noninternal_count", -1);
-	m->incremental = generated_code.find("#define MBG_INCREMENTAL 1") != std::string::npos;
+	m->incremental = generated_code.find("#define MBG_INCREMENTAL 1") != std::string::npos ||
+					 generated_code.find("#define MBG_INCREMENTAL_MANY 1") != std::string::npos;
 	m->integer_rates = generated_code.find("#define MBG_INTEGER_RATES 1") != std::string::npos;
 	m->source = generated_code;
 	// the fast family is compiled now so that errors in the generated code surface here
