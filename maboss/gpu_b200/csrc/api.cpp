@@ -468,7 +468,10 @@ mb_status mb_launch_initialize_random(mb_module mod, void* stream, int n, unsign
 		if (!m.init_random)
 			m.ensure(mb::FAMILY_EPOCH);
 		int per = mb::init_random_per(n);
-		void* a[] = { &n, &seed, &first, &rands, &per };
+		unsigned* jump = m.ctx->xorwow_jump.as<unsigned>();
+		const float* no_istate = nullptr;
+		unsigned* no_states = nullptr;
+		void* a[] = { &n, &seed, &first, &rands, &per, &jump, &no_istate, &no_states, &n };
 		mb::launch(m.init_random, mb::init_random_blocks(n, per), 256, 0, stream_of(m.ctx, stream), a);
 	});
 }

@@ -658,7 +658,10 @@ extern "C" __global__ void __launch_bounds__(128) mb_fused_exact(mb_fused_params
 					rng = static_cast<const curandState*>(P.rands)[t];
 				else
 					curand_init(P.seed, P.first_traj + t, 0ull, &rng);
-				// initial state: one uniform per node in node order (simulation.cu:51-53)
+				if (P.init_states) // drawn by the init launch
+					for (int w = 0; w < state_words; w++)
+						v.S(w) = __ldg(P.init_states + (size_t)w * P.n_traj + t);
+				else // one uniform per node in node order (simulation.cu:51-53)
 				for (int w = 0; w < state_words; w++)
 				{
 					uint32_t sw = 0;
@@ -1052,24 +1055,99 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 
 #if defined(MB_FAMILY_EXACT) || defined(MB_FAMILY_EPOCH)
 // (kept out of the fast family: curand_init's XORWOW skip-ahead tables are megabytes of code)
-// The state of trajectory i is curand_init(seed, first + i, 0) (simulation.cu:23-32). A thread
-// initialises `per` consecutive trajectories: curand_init for the first, then one subsequence jump
-// each (skipahead_sequence(1)), one matrix product instead of the one per digit of the trajectory
-// number that curand_init applies; the states are the same. The host takes per > 1 only when the
-// threads still fill the GPU (the initialisation is latency bound below that).
-extern "C" __global__ void mb_initialize_random(int n, unsigned long long seed, unsigned long long first,
-												 curandState* __restrict__ rands, int per)
+// The state of trajectory i is curand_init(seed, first + i, 0) (simulation.cu:23-32): the seed's state
+// moved on by i subsequences of 2^67 numbers. XORWOW (Marsaglia, "Xorshift RNGs", 2003) is linear over
+// GF(2) in its five words, so a jump is a 160 x 160 bit matrix. A warp holds the matrix of one
+// subsequence in registers (five rows a lane) and applies it to a state that every lane has: per row
+// five and-xors and a parity, and one vote assembles 32 rows into a word: about 40 warp instructions a
+// trajectory, no memory. It does so for `per` consecutive trajectories from the warp's first one, which
+// it reaches by the base-4 digits of the trajectory number (`jump`: for digit position k and digit d the
+// matrix of d 4^k subsequences, [k][d - 1][word of row][row group][lane]; about 8 products of 600 cycles,
+// the latency of their loads). curand_init does one such product per digit and trajectory in one
+// thread. Bound by the vote and parity chain of small batches and by issue slots in large ones. Measured
+// alone: 1e3 trajectories 120 -> 9 us, 1e5 232 -> 21 us, 1e6 466 -> 102 us.
+// With `states`, the warp's lanes also draw the initial states (one uniform per node in node order,
+// simulation.cu:51-53) of 32 trajectories at a time and leave the random states behind them: in the
+// simulation a lane that starts a trajectory would draw them while the other lanes of its warp wait.
+__device__ __forceinline__ void mb_xorwow_jump(unsigned (&x)[5], const unsigned (&rows)[25])
 {
-	const long long id0 = (long long)(blockIdx.x * blockDim.x + threadIdx.x) * per;
+	unsigned y[5];
+#pragma unroll
+	for (int q = 0; q < 5; q++)
+	{
+		unsigned acc = 0;
+#pragma unroll
+		for (int k = 0; k < 5; k++)
+			acc ^= rows[5 * q + k] & x[k];
+		y[q] = __ballot_sync(0xffffffffu, __popc(acc) & 1);
+	}
+#pragma unroll
+	for (int q = 0; q < 5; q++)
+		x[q] = y[q];
+}
+
+__device__ __forceinline__ void mb_xorwow_rows(unsigned (&rows)[25], const unsigned* __restrict__ jump, int matrix)
+{
+#pragma unroll
+	for (int e = 0; e < 25; e++)
+		rows[e] = __ldg(jump + ((size_t)matrix * 25 + e) * 32 + (threadIdx.x & 31));
+}
+
+extern "C" __global__ void __launch_bounds__(MB_INIT_THREADS)
+	mb_initialize_random(int n, unsigned long long seed, unsigned long long first, curandState* __restrict__ rands,
+						 int per, const unsigned* __restrict__ jump, const float* __restrict__ istate,
+						 uint32_t* __restrict__ states, int stride)
+{
+	const int lane = threadIdx.x & 31;
+	const long long id0 = ((long long)blockIdx.x * (MB_INIT_THREADS / 32) + (threadIdx.x >> 5)) * per;
 	if (id0 >= n)
 		return;
 	curandState st;
-	curand_init(seed, first + (unsigned long long)id0, 0ull, &st);
-	rands[id0] = st;
-	for (int k = 1; k < per && id0 + k < n; k++)
+	curand_init(seed, 0ull, 0ull, &st);
+	unsigned x[5], rows[25];
+#pragma unroll
+	for (int k = 0; k < 5; k++)
+		x[k] = st.v[k];
+	unsigned long long e = first + (unsigned long long)id0;
+	for (int k = 0; e; k++, e >>= 2)
 	{
-		skipahead_sequence(1ull, &st);
-		rands[id0 + k] = st;
+		const int d = (int)(e & 3ull);
+		if (d == 0)
+			continue;
+		mb_xorwow_rows(rows, jump, 3 * k + d - 1);
+		mb_xorwow_jump(x, rows);
+	}
+	mb_xorwow_rows(rows, jump, 0);
+	const int count = (int)(n - id0 < per ? n - id0 : per);
+	for (int base = 0; base < count; base += 32)
+	{
+		const int m = count - base < 32 ? count - base : 32;
+		for (int s = 0; s < m; s++)
+		{
+			if (lane == s)
+			{
+#pragma unroll
+				for (int k = 0; k < 5; k++)
+					st.v[k] = x[k];
+			}
+			mb_xorwow_jump(x, rows);
+		}
+		if (lane < m)
+		{
+			const long long id = id0 + base + lane;
+			curandState r = st;
+			if (states)
+				for (int w = 0; w < state_words; w++)
+				{
+					uint32_t sw = 0;
+					const int nb = (w == state_words - 1) ? state_size - 32 * w : 32;
+					for (int b = 0; b < nb; b++)
+						if (curand_uniform(&r) <= __ldg(istate + 32 * w + b))
+							sw |= 1u << b;
+					states[(size_t)w * stride + id] = sw;
+				}
+			rands[id] = r;
+		}
 	}
 }
 #endif

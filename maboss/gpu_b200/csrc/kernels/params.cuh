@@ -37,6 +37,9 @@ struct mb_stats_params
 	unsigned* tail;
 };
 
+// Threads per block of mb_initialize_random.
+constexpr int MB_INIT_THREADS = 256;
+
 // One block's warps take this many neighbouring histogram columns in mb_tail_add.
 constexpr int MB_TAIL_COLS = 8;
 
@@ -53,4 +56,5 @@ struct mb_fused_params
 	unsigned* errors;				 // trajectories stopped because the total rate was not finite
 	void* rands;					 // exact mode: curandState of trajectory t at [t], initialised by a
 									 // separate mb_initialize_random launch, or null (curand_init inline)
+	const unsigned* init_states;	 // exact mode: initial states [word * n_traj + t] that the launch drew, or null
 };

@@ -8,6 +8,7 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -105,6 +106,74 @@ int parse_constexpr(const std::string& src, const std::string& name, int fallbac
 	if (p == std::string::npos)
 		return fallback;
 	return std::atoi(src.c_str() + p + key.size());
+}
+
+// XORWOW's step as 160 x 160 bit matrices over GF(2) (bit 32 k + b: bit b of state word k), squared up to
+// whole subsequences of 2^67 steps: for digit position k and digit d the matrix of d 4^k subsequences,
+// in the order mb_initialize_random reads ([k][d - 1][word of row + 5 row group][lane]). Takes 5 ms, once
+// per process.
+struct bit_matrix
+{
+	std::vector<std::array<unsigned long long, 3>> row = std::vector<std::array<unsigned long long, 3>>(160);
+	bit_matrix operator*(const bit_matrix& o) const
+	{
+		bit_matrix r;
+		for (int j = 0; j < 160; j++)
+		{
+			std::array<unsigned long long, 3> acc{};
+			for (int q = 0; q < 3; q++)
+				for (unsigned long long m = row[j][q]; m; m &= m - 1)
+				{
+					const auto& x = o.row[64 * q + __builtin_ctzll(m)];
+					acc[0] ^= x[0], acc[1] ^= x[1], acc[2] ^= x[2];
+				}
+			r.row[j] = acc;
+		}
+		return r;
+	}
+};
+
+const std::vector<unsigned>& xorwow_jump_table()
+{
+	static const std::vector<unsigned> table = [] {
+		bit_matrix a;
+		auto flip = [&](int to, int from) { a.row[to][from / 64] ^= 1ull << (from % 64); };
+		for (int b = 0; b < 32; b++)
+		{
+			for (int k = 0; k < 4; k++) // x <- y <- z <- w <- v
+				flip(32 * k + b, 32 * (k + 1) + b);
+			// v <- v ^ (v << 4) ^ t ^ (t << 1) with t = x ^ (x >> 2)
+			flip(128 + b, 128 + b);
+			if (b >= 4)
+				flip(128 + b, 128 + b - 4);
+			for (int s = 0; s < 2; s++)
+				if (b >= s)
+				{
+					flip(128 + b, b - s);
+					if (b - s + 2 < 32)
+						flip(128 + b, b - s + 2);
+				}
+		}
+		for (int i = 0; i < 67; i++)
+			a = a * a;
+		std::vector<unsigned> t((size_t)32 * 3 * 25 * 32);
+		for (int k = 0; k < 32; k++)
+		{
+			const bit_matrix a2 = a * a, a3 = a2 * a;
+			const bit_matrix* digit[3] = { &a, &a2, &a3 };
+			for (int d = 0; d < 3; d++)
+				for (int e = 0; e < 25; e++)
+					for (int lane = 0; lane < 32; lane++)
+					{
+						const int word = e % 5, group = e / 5;
+						t[((size_t)(3 * k + d) * 25 + e) * 32 + lane] =
+							(unsigned)(digit[d]->row[32 * group + lane][word / 2] >> (32 * (word % 2)));
+					}
+			a = a2 * a2;
+		}
+		return t;
+	}();
+	return table;
 }
 
 std::mutex cache_mu;
@@ -330,7 +399,16 @@ void module::ensure(int family)
 	if (family == FAMILY_EPOCH_DENSE)
 		get(sim_epoch_dense, "mb_simulate_epoch");
 	if (family != FAMILY_FAST && !init_random)
+	{
+		if (!ctx->xorwow_jump.p)
+		{
+			const std::vector<unsigned>& t = xorwow_jump_table();
+			dbuf b(t.size() * sizeof(unsigned));
+			MB_CUDA(cudaMemcpy(b.p, t.data(), b.bytes, cudaMemcpyHostToDevice));
+			ctx->xorwow_jump = std::move(b);
+		}
 		get(init_random, "mb_initialize_random");
+	}
 	if (!init_state)
 	{
 		get(init_state, "mb_initialize_initial_state");
@@ -910,7 +988,8 @@ namespace {
 
 // Enqueues the fused kernel (and, in exact mode with `rng`, the parallel XORWOW initialisation);
 // returns the number of kernels launched.
-unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long n, cudaStream_t s, void* rng)
+unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long n, cudaStream_t s, void* rng,
+					  unsigned* init_states)
 {
 	if (n > 0xffffffffLL)
 		throw engine_error(MB_ERR_LIMIT, "sample_count above 2^32 - 1");
@@ -933,9 +1012,11 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 	{
 		int cnt = (int)n, per = init_random_per(n);
 		unsigned long long seed = c.seed, first = c.first_traj;
-		void* a[] = { &cnt, &seed, &first, &rng, &per };
+		unsigned* jump = m.ctx->xorwow_jump.as<unsigned>();
+		void* a[] = { &cnt, &seed, &first, &rng, &per, &jump, &P.istate, &init_states, &cnt };
 		launch(m.init_random, init_random_blocks(n, per), 256, 0, s, a);
 		P.rands = rng;
+		P.init_states = init_states;
 		launches++;
 	}
 	int block = c.block;
@@ -1061,7 +1142,9 @@ void run_epochs(module& m, const run_config& c, stats_state& st, long long n, cu
 		unsigned long long seed = c.seed;
 		void* rptr = rbuf.as<char>() + (size_t)offset * sizeof(curandState);
 		int per = init_random_per(cnt);
-		void* a1[] = { &cnt, &seed, &first, &rptr, &per };
+		unsigned* jump = m.ctx->xorwow_jump.as<unsigned>();
+		unsigned* no_states = nullptr;
+		void* a1[] = { &cnt, &seed, &first, &rptr, &per, &jump, &istate, &no_states, &cnt };
 		if (fresh_rng)
 		{
 			launch(m.init_random, init_random_blocks(cnt, per), 256, 0, s, a1);
@@ -1137,7 +1220,11 @@ runner::runner(module& m, const run_config& c) : mod(&m), cfg(c)
 			7u, c.stats_trajectories, c.bin_capacity_log2);
 	st.set_istate(c.istate, s);
 	if (c.mode == MB_MODE_FUSED_EXACT && c.sample_count > 0 && c.sample_count <= max_rng_states)
+	{
 		rng.alloc((size_t)c.sample_count * sizeof(curandState));
+		if (m.incremental && 4 * m.state_words * c.sample_count <= max_init_bytes)
+			init_states.alloc((size_t)4 * m.state_words * c.sample_count);
+	}
 	MB_CUDA(cudaEventCreate(&ev0));
 	MB_CUDA(cudaEventCreate(&ev1));
 	MB_CUDA(cudaStreamSynchronize(s));
@@ -1166,7 +1253,7 @@ void runner::launch(cudaStream_t s)
 		run_epochs(*mod, cfg, st, cfg.sample_count, s, epochs, launches);
 	else
 	{
-		launches = launch_fused(*mod, cfg, st, cfg.sample_count, s, rng.p);
+		launches = launch_fused(*mod, cfg, st, cfg.sample_count, s, rng.p, init_states.as<unsigned>());
 		epochs = 1;
 	}
 	MB_CUDA(cudaEventRecord(ev1, s));

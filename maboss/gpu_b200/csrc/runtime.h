@@ -30,18 +30,18 @@ struct engine_error : std::runtime_error
 void cuda_throw(cudaError_t e, const char* what);
 #define MB_CUDA(x) ::mb::cuda_throw((x), #x)
 
-// mb_initialize_random: trajectories initialised per thread (consecutive ones, by subsequence jumps)
-// and the grid of 256-thread blocks for n trajectories. Up to 8 per thread, as long as the threads
-// still number 148 SMs x 512; below that the initialisation is latency bound and each thread takes
-// one.
+// mb_initialize_random: consecutive trajectories per warp and the grid for n trajectories. One per warp until
+// the chip has 32 warps an SM to hide the latency of the jumps to each warp's first trajectory, then as
+// many as keep that number of warps, up to 128 (the jumps are then a twentieth of the work).
 inline int init_random_per(long long n)
 {
-	const long long per = n / (148LL * 512);
-	return per < 1 ? 1 : per > 8 ? 8 : (int)per;
+	const long long warps = 148LL * 32, per = (n + warps - 1) / warps;
+	return per < 1 ? 1 : per > 128 ? 128 : (int)per;
 }
 inline unsigned init_random_blocks(long long n, int per)
 {
-	return (unsigned)((n + 256LL * per - 1) / (256LL * per));
+	const long long block = (long long)per * (MB_INIT_THREADS / 32);
+	return (unsigned)((n + block - 1) / block);
 }
 
 // Device memory owned by the runtime.
@@ -75,6 +75,7 @@ struct context
 	int sm_count = 0;
 	int cc_major = 0, cc_minor = 0;
 	cudaStream_t stream = nullptr; // owned, non-blocking
+	dbuf xorwow_jump; // jump matrices of mb_initialize_random, uploaded with the first module that has it
 	explicit context(int device);
 	~context();
 };
@@ -319,6 +320,10 @@ struct runner
 	unsigned launches = 0; // engine kernels enqueued by the last launch()
 	dbuf rng;			   // exact mode: XORWOW states of every trajectory (empty above max_rng_states)
 	static constexpr long long max_rng_states = 1LL << 24;
+	// incremental exact mode: initial states of every trajectory (empty where they take more than 1 GB:
+	// the kernel then draws them itself)
+	dbuf init_states;
+	static constexpr long long max_init_bytes = 1LL << 30;
 	runner(module& m, const run_config& c);
 	~runner();
 	void launch(cudaStream_t s);
