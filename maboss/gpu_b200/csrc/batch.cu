@@ -433,7 +433,9 @@ void batch_engine::set_shape(prepared& ps, int block, int per_sm)
 																 (228 * 1024)))
 										  : -1;
 	MB_CUDA(cudaFuncSetAttribute(ps.fn, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-	const unsigned long long needed = (ps.B->total + block - 1) / block;
+	ps.B->lanes = lanes_per_warp((long long)std::min<unsigned long long>(ps.B->total, 1ull << 40), ctx->sm_count);
+	const unsigned long long per_block = (unsigned long long)(block / 32) * ps.B->lanes;
+	const unsigned long long needed = (ps.B->total + per_block - 1) / per_block;
 	ps.block = block;
 	ps.per_sm = per_sm;
 	ps.smem = smem;

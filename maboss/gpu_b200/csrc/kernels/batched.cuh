@@ -60,6 +60,7 @@ struct mb_batch_params
 	int max_W;			  // shared memory rows per lane
 	int P;				  // gradient parameters (rows of gradient scratch), 0 = none
 	unsigned long long total;
+	int lanes;			  // lanes of each warp that take trajectories (fewer than 32 in small runs)
 	unsigned long long seed;
 	unsigned long long* next;
 	unsigned* errors;
@@ -358,7 +359,7 @@ __device__ void mbb_body(const mb_batch_params& B)
 	int acc_var = -1; // variant whose accumulators `acc` refers to
 	mbb_cot_cache cc;
 
-	bool working = true, running = false;
+	bool working = lane < B.lanes, running = false;
 	int vi = 0; // current variant of this lane
 	unsigned long long gs[MBB_GROUPS];
 	unsigned long long total = 0;

@@ -197,7 +197,7 @@ __device__ __forceinline__ void mb_fused_body(const mb_fused_params& P)
 	unsigned long long trans = 0;
 	mb_win_acc acc;
 	mb_acc_init(acc);
-	for (;;)
+	for (; (int)(threadIdx.x & 31) < P.lanes;)
 	{
 		const unsigned long long t = atomicAdd(P.next_traj, 1ull);
 		if (t >= P.n_traj)
@@ -634,7 +634,7 @@ extern "C" __global__ void __launch_bounds__(128) mb_fused_exact(mb_fused_params
 	unsigned long long trans = 0;
 	mb_win_acc acc;
 	mb_acc_init(acc);
-	bool working = true, running = false;
+	bool working = lane < P.lanes, running = false;
 	mb_idx_t idx = 0;
 	float time = 0.f;
 	int slot = 1;
@@ -804,7 +804,7 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 	mb_acc_init(acc);
 
 	// per-lane trajectory registers
-	bool working = true;  // the work counter is not exhausted for this lane
+	bool working = lane < P.lanes; // the work counter is not exhausted for this lane
 	bool running = false; // the lane holds a trajectory
 	unsigned long long gs[MB_GROUPS]; // inclusive prefix sums of the groups' rate sums
 	unsigned long long total = 0;

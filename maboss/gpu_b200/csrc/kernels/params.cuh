@@ -50,6 +50,7 @@ struct mb_fused_params
 	unsigned long long seed;		 // seed_pseudorandom
 	unsigned long long first_traj;	 // global id of trajectory 0 of this launch (RNG subsequence)
 	unsigned n_traj;				 // trajectories of this launch
+	int lanes;						 // lanes of each warp that take trajectories (fewer than 32 in small runs)
 	int traj_len;					 // epoch length L emulated in exact mode (0 = none)
 	unsigned long long* next_traj;	 // work counter (zeroed by the host)
 	unsigned long long* transitions; // executed simulate iterations

@@ -1042,7 +1042,8 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 	cu_throw(drv().FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, carve),
 			 "cuFuncSetAttribute");
 	const int per_sm = c.blocks_per_sm > 0 ? c.blocks_per_sm : occupancy_blocks(f, block, smem);
-	const long long needed = (n + block - 1) / block;
+	P.lanes = lanes_per_warp(n, m.ctx->sm_count);
+	const long long per_block = (long long)(block / 32) * P.lanes, needed = (n + per_block - 1) / per_block;
 	const unsigned grid = (unsigned)std::max(1LL, std::min<long long>(needed, (long long)per_sm * m.ctx->sm_count));
 	void* args[] = { &P };
 	launch(f, grid, block, smem, s, args);

@@ -30,6 +30,18 @@ struct engine_error : std::runtime_error
 void cuda_throw(cudaError_t e, const char* what);
 #define MB_CUDA(x) ::mb::cuda_throw((x), #x)
 
+// Lanes of each warp that take trajectories in a run of n. A warp's lanes run their own trajectories, so
+// a step of 32 of them costs two to three times the instructions of a step of one, and a run too small
+// for two warps on each scheduler waits on latencies: it is spread over 8 warps an SM with fewer lanes
+// each. Kernel time before -> after (with 12 warps an SM), us: 32-node example model, exact mode, 1e3
+// trajectories 1255 -> 411 (408), 1e4 1360 -> 645 (630); 50 nodes fast 1e3 687 -> 363 (365), 1e4 734 ->
+// 617 (652), 3e4 799 -> 729 (768); 87-node example model fast 3e4 4804 -> 4585 (4969: slower).
+inline int lanes_per_warp(long long n, int sm_count)
+{
+	const long long warps = 8LL * sm_count, lanes = (n + warps - 1) / warps;
+	return lanes < 1 ? 1 : lanes > 32 ? 32 : (int)lanes;
+}
+
 // mb_initialize_random: consecutive trajectories per warp and the grid for n trajectories. One per warp until
 // the chip has 32 warps an SM to hide the latency of the jumps to each warp's first trajectory, then as
 // many as keep that number of warps, up to 128 (the jumps are then a twentieth of the work).
