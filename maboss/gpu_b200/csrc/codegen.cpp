@@ -1,5 +1,6 @@
 // Model -> CUDA source. See codegen.h.
 #include "codegen.h"
+#include "gates.h"
 
 #include <algorithm>
 #include <cmath>
@@ -417,6 +418,93 @@ void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 		if (last_in_word)
 			ss << "    }" << std::endl;
 	}
+	ss << "}" << std::endl;
+}
+
+// Tables of the lockstep kernels: the network's gates (gates.h) as {byte offset of a | of b << 16 | or <<
+// 31, byte offset of c | of d << 16 | invert << 31}, and, for models whose positive rates take at most
+// three values, the unstable nodes of each value as masks (their sums are then population counts).
+void emit_gates(std::ostream& ss, const model_t& m, const model_layout& L)
+{
+	if (!L.incremental_ok)
+		return;
+	const gate_network net = build_gates(m);
+	if (!net.ok)
+		return;
+	ss << std::endl << "// ---- lockstep kernels" << std::endl;
+	ss << "#define MBG_GATES 1" << std::endl;
+	ss << "constexpr int mbg_gate_rounds = " << net.rounds << ";" << std::endl;
+	ss << "constexpr int mbg_gate_words = " << net.words << ";" << std::endl;
+	std::vector<std::string> g2;
+	for (const gate& g : net.gates)
+	{
+		const unsigned x = (unsigned)g.in[0] * 4 | (unsigned)g.in[1] * 4 << 16 | (g.is_or ? 1u << 31 : 0u);
+		const unsigned y = (unsigned)g.in[2] * 4 | (unsigned)g.in[3] * 4 << 16 | (g.invert ? 1u << 31 : 0u);
+		g2.push_back("{" + std::to_string(x) + "u, " + std::to_string(y) + "u}");
+	}
+	emit_array(ss, "uint2", "mbg_gates", g2);
+	std::vector<unsigned> ni(L.state_words, 0u);
+	for (int i : L.noninternal_nodes)
+		ni[i / 32] |= 1u << (i % 32);
+	ss << "__device__ __forceinline__ constexpr uint32_t mbg_ni_mask(int w)" << std::endl << "{" << std::endl << "    return ";
+	for (int w = 0; w < L.state_words; w++)
+		ss << "w == " << w << " ? " << ni[w] << "u : ";
+	ss << "0u;" << std::endl << "}" << std::endl;
+	// the non-internal nodes' rates in their order, 0 for stable nodes
+	ss << "template <class V, class F>" << std::endl;
+	ss << "__device__ __forceinline__ void mbg_ni_each_rate(const V& v, F f)" << std::endl << "{" << std::endl;
+	for (int i : L.noninternal_nodes)
+	{
+		const unsigned bit = 1u << (i % 32);
+		ss << "    f((v.U(" << i / 32 << ") & " << bit << "u) ? (v.S(" << i / 32 << ") & " << bit << "u) ? "
+		   << flit(L.down[i]) << " : " << flit(L.up[i]) << " : 0.f);" << std::endl;
+	}
+	ss << "}" << std::endl;
+	std::vector<float> values;
+	double sum = 0;
+	for (int i = 0; i < L.state_size; i++)
+	{
+		for (float r : { L.up[i], L.down[i] })
+			if (r > 0.f && std::find(values.begin(), values.end(), r) == values.end())
+				values.push_back(r);
+		sum += std::max(L.up[i], L.down[i]);
+	}
+	// sums of rates that are whole multiples of some 2^-k, at most 2^24 of them, have no rounding in fp32, so
+	// they can be taken in any order
+	int low = 1000;
+	for (float r : values)
+	{
+		int e;
+		const double f = std::frexp((double)r, &e);
+		low = std::min(low, e - 24 + __builtin_ctz((unsigned)std::ldexp(f, 24)));
+	}
+	if (values.empty() || values.size() > 3 || !std::isfinite(sum) || std::ldexp(sum, -low) > 16777216.0)
+		return;
+	ss << "#define MBG_RATE_CLASSES " << values.size() << std::endl;
+	ss << "__device__ __forceinline__ constexpr float mbg_class_rate(int d)" << std::endl << "{" << std::endl << "    return ";
+	for (size_t d = 0; d < values.size(); d++)
+		ss << "d == " << d << " ? " << flit(values[d]) << " : ";
+	ss << "0.f;" << std::endl << "}" << std::endl;
+	ss << "__device__ __forceinline__ constexpr uint32_t mbg_class_q(int d)" << std::endl << "{" << std::endl << "    return ";
+	for (size_t d = 0; d < values.size(); d++)
+		ss << "d == " << d << " ? "
+		   << (unsigned)std::min(std::nearbyint((double)values[d] * std::ldexp(1.0, L.rate_shift)), 4294967295.0) << "u : ";
+	ss << "0u;" << std::endl << "}" << std::endl;
+	// f(w, d, the unstable nodes of word w whose rate has value d)
+	ss << "template <class V, class F>" << std::endl;
+	ss << "__device__ __forceinline__ void mbg_class_each(const V& v, F f)" << std::endl << "{" << std::endl;
+	for (int w = 0; w < L.state_words; w++)
+		for (size_t d = 0; d < values.size(); d++)
+		{
+			unsigned up = 0, down = 0;
+			for (int i = 32 * w; i < std::min(L.state_size, 32 * w + 32); i++)
+			{
+				up |= L.up[i] == values[d] ? 1u << (i % 32) : 0u;
+				down |= L.down[i] == values[d] ? 1u << (i % 32) : 0u;
+			}
+			ss << "    f(" << w << ", " << d << ", v.U(" << w << ") & ((v.S(" << w << ") & " << down << "u) | (~v.S(" << w
+			   << ") & " << up << "u)));" << std::endl;
+		}
 	ss << "}" << std::endl;
 }
 
@@ -999,6 +1087,7 @@ std::string generate_code(const model_t& m)
 	ss << "    return h > 0.f ? h : 0.f;" << std::endl << "}" << std::endl;
 
 	emit_incremental_tables(ss, L);
+	emit_gates(ss, m, L);
 	return ss.str();
 }
 

@@ -340,6 +340,7 @@ std::unique_ptr<module> compile_module(context& ctx, const std::string& generate
 	m->incremental = generated_code.find("#define MBG_INCREMENTAL 1") != std::string::npos ||
 					 generated_code.find("#define MBG_INCREMENTAL_MANY 1") != std::string::npos;
 	m->integer_rates = generated_code.find("#define MBG_INTEGER_RATES 1") != std::string::npos;
+	m->gate_words = parse_constexpr(generated_code, "mbg_gate_words", 0);
 	m->source = generated_code;
 	// the fast family is compiled now so that errors in the generated code surface here
 	m->ensure(FAMILY_FAST);
@@ -1023,15 +1024,14 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 	size_t smem = st.h_smem();
 	if (c.mode == MB_MODE_FUSED_EXACT ? m.incremental : m.fast_incremental())
 	{
-		// per thread in shared memory: state words, unstable masks and word rate sums
-		const size_t per_word = 12;
+		// per thread in shared memory: state words, unstable masks and word rate sums; or per warp its array
 		constexpr size_t max_smem = 227 * 1024;
 		block = std::min(block, 128);
-		while (block > 32 && per_word * m.state_words * block + smem > max_smem)
+		while (block > 32 && m.fused_smem(block) + smem > max_smem)
 			block -= 32;
-		if (per_word * m.state_words * block + smem > max_smem)
+		if (m.fused_smem(block) + smem > max_smem)
 			throw engine_error(MB_ERR_LIMIT, "model too large for the incremental kernel's shared memory");
-		smem += per_word * m.state_words * block;
+		smem += m.fused_smem(block);
 	}
 	// an explicit block count per SM also fixes the shared-memory carve-out to what those blocks need
 	// (+1 KB reserved per block), leaving the rest of the SM's 256 KB of L1/shared memory to L1
@@ -1283,7 +1283,7 @@ std::vector<tuned_shape> autotune(module& m, const run_config& c)
 	const std::vector<int> blocks = incr ? std::vector<int>{ 128, 96, 64 } : std::vector<int>{ 256, 128 };
 	for (int block : blocks)
 	{
-		size_t smem = incr ? (size_t)12 * m.state_words * block : 0;
+		size_t smem = incr ? m.fused_smem(block) : 0;
 		if (smem > 227 * 1024)
 			continue;
 		MB_CUDA(cudaSetDevice(m.ctx->device));

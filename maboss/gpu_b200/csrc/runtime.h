@@ -119,6 +119,13 @@ struct module
 	bool incremental = false;	// @logic-form model: exact and epoch modes use the incremental kernels (generated MBG_INCREMENTAL)
 	bool integer_rates = false; // fast mode's incremental kernel too (generated MBG_INTEGER_RATES), else its dense kernel
 	bool fast_incremental() const { return incremental && integer_rates; }
+	// words of a warp's array in the lockstep kernels (generated MBG_GATES), 0: the incremental kernels
+	int gate_words = 0;
+	// dynamic shared memory of a block of a fused incremental kernel, without the entropy sums
+	size_t fused_smem(int block) const
+	{
+		return gate_words ? (size_t)4 * gate_words * (block / 32) : (size_t)12 * state_words * block;
+	}
 	bool has_layout = false; // compiled from a model (full layout known)
 	model_layout layout;
 	std::string source; // generated model source that was compiled with the engine
