@@ -1793,7 +1793,121 @@ extern "C" __global__ void mb_initialize_initial_state(int n, int stride, const 
 }
 
 #ifdef MB_FAMILY_EPOCH
-#if defined(MBG_INCREMENTAL) && !defined(MB_EPOCH_DENSE)
+#if defined(MBG_INCREMENTAL) && defined(MBG_GATES) && !defined(MB_EPOCH_DENSE)
+// One epoch of at most L-1 recorded steps per trajectory (simulation.cu:77-164) on lockstep logic: the exact
+// algorithm, each step written to the SoA trajectory buffer; the warp's trajectories are at the same slot,
+// so its stores are contiguous. Shared memory: the warps' arrays. 1e5 trajectories of the 87-node example
+// model, whole run with the buffers kept: 18 to 28 ms before (varying with the allocations), 6.0 ms now.
+extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS)
+	mb_simulate_epoch(int n, int stride, int L, uint32_t* __restrict__ last_states, float* __restrict__ last_times,
+					  curandState* __restrict__ rands, uint32_t* __restrict__ traj_states,
+					  float* __restrict__ traj_times, float* __restrict__ traj_h, uint8_t* __restrict__ statuses,
+					  unsigned long long* __restrict__ transitions)
+{
+	extern __shared__ __align__(16) uint32_t mb_smem_u32[];
+	uint32_t* ns = mb_lock_words(mb_smem_u32);
+	const int id = blockIdx.x * blockDim.x + threadIdx.x;
+	const bool active = id < n;
+	bool running = active;
+	mb_lock v;
+	float q[MB_LW];
+#pragma unroll
+	for (int w = 0; w < MB_LW; w++)
+	{
+		v.s[w] = active ? last_states[(size_t)w * stride + id] : 0u;
+		v.u[w] = 0u;
+		q[w] = 0.f;
+	}
+	curandState rng;
+	float time = 0.f;
+	if (active)
+	{
+		rng = rands[id];
+		time = last_times[id];
+		traj_times[id] = time;
+	}
+	trajectory_status status = trajectory_status::CONTINUE;
+	unsigned long long trans = 0;
+	float h_cache = 0.f;
+	int step = 1, j = -1;
+	bool first = true;
+	mb_lock_fill(ns, v);
+	while (__any_sync(0xffffffffu, running))
+	{
+		uint32_t u[MB_LW];
+		mb_lock_unstable(ns, u);
+		const bool ni_changed = mb_lock_ni_changed(v, u, j) || first;
+		first = false;
+		if (running)
+		{
+			mb_lock_exact_sums(v, u, j, q);
+			j = -1;
+			const float total = q[MB_LW - 1];
+			float h = 0.f;
+			if (isinf(total))
+			{
+				// an infinite total rate gives zero waiting times forever: end the trajectory
+				time = max_time;
+				running = false;
+			}
+			else
+			{
+				if (total == 0.f)
+				{
+					status = trajectory_status::FIXED_POINT;
+					time = max_time;
+				}
+				else
+				{
+					if (discrete_time)
+					{
+						time += time_tick;
+						time = max_time - time_tick < time ? max_time : time;
+					}
+					else
+						time += -logf(curand_uniform(&rng)) / total;
+					time = fminf(time, max_time);
+					if (ni_changed)
+						h_cache = mb_lock_exact_entropy(v);
+					h = h_cache;
+				}
+#pragma unroll
+				for (int w = 0; w < MB_LW; w++)
+					traj_states[((size_t)step * state_words + w) * stride + id] = v.s[w];
+				traj_times[(size_t)step * stride + id] = time;
+				traj_h[(size_t)step * stride + id] = h;
+				trans += (time != 0.f) ? 1ull : 0ull;
+				step++;
+				if (time >= max_time || step >= L)
+					running = false;
+				else
+				{
+					j = mb_lock_exact_select(v, q, curand_uniform(&rng) * total);
+					mb_lock_flip(ns, v, j);
+				}
+			}
+		}
+	}
+	if (active)
+	{
+		for (int s = step; s < L; s++) // empty slots carry the zero-time sentinel
+			traj_times[(size_t)s * stride + id] = 0.f;
+#pragma unroll
+		for (int w = 0; w < MB_LW; w++)
+			last_states[(size_t)w * stride + id] = v.s[w];
+		rands[id] = rng;
+		last_times[id] = time;
+		if (status != trajectory_status::FIXED_POINT)
+			status = (time >= max_time) ? trajectory_status::FINISHED : trajectory_status::CONTINUE;
+		statuses[id] = (uint8_t)status;
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+		trans += __shfl_down_sync(0xffffffffu, trans, o);
+	if ((threadIdx.x & 31) == 0 && trans)
+		atomicAdd(transitions, trans);
+}
+#elif defined(MBG_INCREMENTAL) && !defined(MB_EPOCH_DENSE)
 // One epoch of at most L-1 recorded steps per trajectory (simulation.cu:77-164) for models whose
 // rates all have the @logic form: the exact algorithm on incremental unstable sets (the same
 // results as the dense per-step evaluation below), each step written to the SoA trajectory buffer

@@ -356,6 +356,7 @@ std::unique_ptr<module> compile_batch_module(context& ctx, const std::string& ge
 	m->noninternal_count = parse_constexpr(generated_code, "mbg_noninternal_count", -1);
 	m->incremental = generated_code.find("#define MBG_INCREMENTAL 1") != std::string::npos;
 	m->integer_rates = generated_code.find("#define MBG_INTEGER_RATES 1") != std::string::npos;
+	m->gate_words = parse_constexpr(generated_code, "mbg_gate_words", 0);
 	m->source = generated_code;
 	return m;
 }
@@ -1073,12 +1074,12 @@ void simulate_epoch(module& m, bool dense, cudaStream_t s, int n, int stride, in
 		launch(m.sim_epoch, (n + 255) / 256, 256, 0, s, a);
 		return;
 	}
-	// per thread in shared memory: state words, unstable masks, word-end running sums
+	// per thread in shared memory: state words, unstable masks, word-end running sums; or per warp its array
 	constexpr size_t max_smem = 227 * 1024;
 	int block = 128;
-	while (block > 32 && (size_t)12 * m.state_words * block > max_smem)
+	while (block > 32 && m.fused_smem(block) > max_smem)
 		block -= 32;
-	const size_t smem = (size_t)12 * m.state_words * block;
+	const size_t smem = m.fused_smem(block);
 	if (smem > max_smem)
 		throw engine_error(MB_ERR_LIMIT, "model too large for the incremental epoch kernel's shared memory");
 	launch(m.sim_epoch, (n + block - 1) / block, block, smem, s, a);
@@ -1119,8 +1120,8 @@ void partition(module& m, cudaStream_t s, int n, int stride, const unsigned char
 
 namespace {
 
-void run_epochs(module& m, const run_config& c, stats_state& st, long long n, cudaStream_t s, int& epochs,
-				unsigned& launches)
+void run_epochs(module& m, const run_config& c, stats_state& st, epoch_buffers& E, long long n, cudaStream_t s,
+				int& epochs, unsigned& launches)
 {
 	const int W = m.state_words;
 	const int L = std::max(2, c.traj_len);
@@ -1129,10 +1130,25 @@ void run_epochs(module& m, const run_config& c, stats_state& st, long long n, cu
 	m.ensure(c.mode == MB_MODE_EPOCH_DENSE ? FAMILY_EPOCH_DENSE : FAMILY_EPOCH);
 	const long long Bll = std::min<long long>(std::max(1, c.batch_limit), n);
 	const int B = (int)Bll;
-	dbuf st0((size_t)W * B * 4), st1((size_t)W * B * 4), t0((size_t)B * 4), t1((size_t)B * 4);
-	dbuf r0((size_t)B * sizeof(curandState)), r1((size_t)B * sizeof(curandState));
-	dbuf ts((size_t)L * W * B * 4), tt((size_t)L * B * 4), th((size_t)L * B * 4), stat((size_t)B);
-	dbuf scratch(256 + partition_scratch_bytes(B));
+	if (E.batch != B) // (a runner's L and W do not change)
+	{
+		E = epoch_buffers();
+		for (int k = 0; k < 2; k++)
+		{
+			E.states[k].alloc((size_t)W * B * 4);
+			E.times[k].alloc((size_t)B * 4);
+			E.rands[k].alloc((size_t)B * sizeof(curandState));
+		}
+		E.traj_states.alloc((size_t)L * W * B * 4);
+		E.traj_times.alloc((size_t)L * B * 4);
+		E.traj_h.alloc((size_t)L * B * 4);
+		E.statuses.alloc((size_t)B);
+		E.scratch.alloc(256 + partition_scratch_bytes(B));
+		E.batch = B;
+		E.bytes = (size_t)L * (W + 2) * B * 4;
+	}
+	dbuf &st0 = E.states[0], &st1 = E.states[1], &t0 = E.times[0], &t1 = E.times[1], &r0 = E.rands[0], &r1 = E.rands[1];
+	dbuf &ts = E.traj_states, &tt = E.traj_times, &th = E.traj_h, &stat = E.statuses, &scratch = E.scratch;
 	unsigned long long* trans = st.transitions();
 	float* istate = st.istate.as<float>();
 
@@ -1251,7 +1267,11 @@ void runner::launch(cudaStream_t s)
 	epochs = 0;
 	launches = 0;
 	if (cfg.mode == MB_MODE_EPOCH || cfg.mode == MB_MODE_EPOCH_DENSE)
-		run_epochs(*mod, cfg, st, cfg.sample_count, s, epochs, launches);
+	{
+		run_epochs(*mod, cfg, st, epoch, cfg.sample_count, s, epochs, launches);
+		if (epoch.bytes > max_epoch_bytes)
+			epoch = epoch_buffers(); // (the last epoch has been waited for)
+	}
 	else
 	{
 		launches = launch_fused(*mod, cfg, st, cfg.sample_count, s, rng.p, init_states.as<unsigned>());

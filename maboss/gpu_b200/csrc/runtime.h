@@ -327,6 +327,14 @@ struct stats_state
 	std::unique_ptr<result> finalize(long long n_traj, cudaStream_t s);
 };
 
+// Device buffers of the epoch modes' batch (states, times, random states twice, trajectory slots).
+struct epoch_buffers
+{
+	dbuf states[2], times[2], rands[2], traj_states, traj_times, traj_h, statuses, scratch;
+	int batch = 0;
+	size_t bytes = 0;
+};
+
 // A run whose device buffers are allocated once: launch() zeroes the accumulators and enqueues the
 // simulation on a stream without synchronising (fused modes), collect() copies the results back.
 struct runner
@@ -343,6 +351,10 @@ struct runner
 	// the kernel then draws them itself)
 	dbuf init_states;
 	static constexpr long long max_init_bytes = 1LL << 30;
+	// epoch modes: kept for the next launch where they take at most 4 GB (allocating and freeing the 0.2 GB of
+	// 1e5 trajectories of the 87-node example model took 9 to 20 ms a run), else given back after each run
+	epoch_buffers epoch;
+	static constexpr size_t max_epoch_bytes = 4ull << 30;
 	runner(module& m, const run_config& c);
 	~runner();
 	void launch(cudaStream_t s);
