@@ -119,6 +119,7 @@ private:
 		bool grad = false;
 		std::unique_ptr<mb_batch_params> B; // the kernel's parameter block
 		const void* fn = nullptr;
+		size_t smem_per_warp = 0; // the lockstep kernels' arrays
 		size_t smem_per_thread = 0, smem = 0;
 		int block = 0, per_sm = 0;
 		unsigned grid = 0;

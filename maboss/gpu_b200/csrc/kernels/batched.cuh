@@ -704,12 +704,301 @@ struct mbb_net_static
 		mbg_ni_rate_sums_var(v, var.rate, var.rlog, t, tl);
 	}
 };
+#ifdef MBG_GATES
+// The batched algorithm on lockstep logic (networks of at most 256 nodes, kernels/engine.cuh): the same random
+// numbers, rates, choices and order of the score's updates as mbb_body. Shared memory: the warps' arrays,
+// then the gradient's A_p and D_p of every thread. Forward and gradient of the 50-node network with 40
+// parameters, 1e6 trajectories, end to end 31.6 -> 25.0 ms.
+template <bool GRAD>
+__device__ void mbb_lock_body(const mb_batch_params& B)
+{
+	extern __shared__ __align__(16) uint32_t mbb_smem[];
+	const int bs = blockDim.x, lane = threadIdx.x & 31;
+	const int P = GRAD ? B.P : 0;
+	constexpr bool discrete = discrete_time;
+	constexpr float tick = time_tick, end_time = ::max_time;
+	uint32_t* ns = mb_lock_words(mbb_smem);
+	mbb_lane g; // the gradient's rows (the states are in v)
+	float* gbase = reinterpret_cast<float*>(mbb_smem + (bs >> 5) * mbg_gate_words);
+	g.stride = bs;
+	g.gS = gbase + threadIdx.x;
+	g.gD = gbase + (size_t)P * bs + threadIdx.x;
+	g.gstride = B.gstride;
+	g.gR = GRAD ? B.gmem + blockIdx.x * bs + threadIdx.x : nullptr;
+	double C1 = 0.0, C2 = 0.0; // continuous-time gradient running sums of the lane's trajectory
+	for (int p = 0; p < P; p++)
+	{
+		g.GS(p) = 0.f;
+		g.GD(p) = 0.f;
+		*g.GR(p) = 0.0;
+	}
+	mb_win_acc acc;
+	mb_acc_init(acc);
+	int acc_var = -1; // variant whose accumulators `acc` refers to
+	mbb_cot_cache cc;
+
+	bool working = lane < B.lanes, running = false;
+	int vi = 0; // current variant of this lane
+	mb_lock v;
+	uint32_t q[MB_LW];
+#pragma unroll
+	for (int w = 0; w < MB_LW; w++)
+		v.s[w] = v.u[w] = q[w] = 0u;
+	uint32_t idx = 0;
+	float time = 0.f, h = 0.f;
+	int j = -1;
+	unsigned long long trans = 0;
+	curandStatePhilox4_32_10_t rng;
+
+	while (__any_sync(0xffffffffu, working || running))
+	{
+		unsigned long long t = 0;
+		int tv = 0;
+		bool starting = false;
+		if (working && !running)
+		{
+			t = atomicAdd(B.next, 1ull);
+			if (t < B.total)
+			{
+				// variant of work item t (variants are laid out back to back)
+				int lo = 0, hi = B.n_vars - 1;
+				while (lo < hi)
+				{
+					const int mid = (lo + hi + 1) >> 1;
+					if (B.vars[mid].begin <= t)
+						lo = mid;
+					else
+						hi = mid - 1;
+				}
+				tv = lo;
+				starting = true;
+			}
+			else
+				working = false;
+		}
+		unsigned pending = __ballot_sync(0xffffffffu, starting);
+		if (pending)
+		{
+			uint32_t* words = ns + 64 * MB_LW + 2; // (the gates' words)
+			while (pending)
+			{
+				const int src = __ffs(pending) - 1;
+				pending &= pending - 1u;
+				const unsigned long long ts = __shfl_sync(0xffffffffu, t, src);
+				const mb_variant& var = B.vars[__shfl_sync(0xffffffffu, tv, src)];
+				mb_philox_initial_state(B.seed, var.first_traj + (ts - var.begin), state_size, var.istate,
+										[&](int w, uint32_t word) {
+											if (lane == 0)
+												words[w] = word;
+										});
+				__syncwarp();
+				if (lane == src)
+				{
+#pragma unroll
+					for (int w = 0; w < MB_LW; w++)
+						v.s[w] = words[w];
+				}
+				__syncwarp();
+			}
+			if (starting)
+			{
+				vi = tv;
+				const mb_variant& var = B.vars[vi];
+				curand_init(B.seed, var.first_traj + (t - var.begin), (unsigned long long)((state_size + 3) & ~3), &rng);
+#pragma unroll
+				for (int w = 0; w < MB_LW; w++)
+					v.u[w] = q[w] = 0u;
+				idx = get_non_internal_index(v.s);
+				time = 0.f;
+				j = -1;
+				C1 = C2 = 0.0;
+				running = true;
+				if (acc_var != vi)
+				{
+					if (acc_var >= 0)
+					{
+						mb_acc_flush(acc, B.vars[acc_var].st, B.vars[acc_var].st.win_h);
+						if (GRAD)
+							mbb_grad_emit(B.vars[acc_var], g, P);
+					}
+					acc_var = vi;
+					cc.w = -1;
+				}
+			}
+			mb_lock_fill(ns, v);
+		}
+		uint32_t n[MB_LW];
+		mb_lock_unstable(ns, n);
+		const bool ni_changed = mb_lock_ni_changed(v, n, j) || starting;
+		if (running)
+		{
+			const mb_variant& var = B.vars[vi];
+			unsigned long long total = 0;
+#pragma unroll
+			for (int w = 0; w < MB_LW; w++)
+			{
+				uint32_t c = mb_lock_changed(v, n, w, j);
+				const uint32_t fb = j >= 0 && (j >> 5) == w ? 1u << (j & 31) : 0u;
+				while (c)
+				{
+					const int b = __ffs(c) - 1;
+					c &= c - 1u;
+					const uint2 qq = __ldg(var.q + 32 * w + b);
+					const uint32_t now = (v.s[w] >> b) & 1u, was = now ^ ((fb >> b) & 1u);
+					const bool is_u = (n[w] >> b) & 1u, was_u = (v.u[w] >> b) & 1u;
+					q[w] += is_u ? (now ? qq.y : qq.x) : 0u;
+					q[w] -= was_u ? (was ? qq.y : qq.x) : 0u;
+					if (GRAD)
+					{
+						if (was_u)
+							mbb_grad_active(var, g, 32 * w + b, (int)was, -1.f, time, discrete, C1, C2);
+						if (is_u)
+							mbb_grad_active(var, g, 32 * w + b, (int)now, 1.f, time, discrete, C1, C2);
+					}
+				}
+				v.u[w] = n[w];
+				total += q[w];
+			}
+			j = -1;
+			if (ni_changed)
+			{
+				float rt = 0.f, rl = 0.f;
+				mbg_ni_rate_sums_var(v, var.rate, var.rlog, rt, rl);
+				h = 0.f;
+				if (rt > 0.f)
+				{
+					const float x = log2f(rt) - rl / rt;
+					h = x > 0.f ? x : 0.f;
+				}
+			}
+			if (total == 0)
+			{
+				// a fixed point: the state stays until max_time
+				running = false;
+				mbb_record<GRAD>(var, g, P, acc, idx, time, end_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
+				atomicAdd(var.st.final_cnt + idx, 1u);
+				uint32_t st[MB_LW]; // (a copy: v.s stays in registers)
+#pragma unroll
+				for (int w = 0; w < MB_LW; w++)
+					st[w] = v.s[w];
+				mb_fixed_insert_rt(var.st, st, MB_LW);
+				if (GRAD)
+					mbb_grad_end(g, P, discrete, C1, C2);
+				atomicAdd(var.transitions, trans + 1);
+				trans = 0;
+			}
+			else
+			{
+				const uint4 rb = curand4(&rng);
+				const float a0 = (float)total * (1.0f / (float)(1u << var.rate_shift));
+				float tn;
+				if (discrete)
+				{
+					tn = time + tick;
+					tn = end_time - tick < tn ? end_time : tn;
+				}
+				else
+				{
+					const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
+					tn = time + -logf(u) / a0;
+				}
+				tn = fminf(tn, end_time);
+				trans += (tn != 0.f) ? 1ull : 0ull;
+				mbb_record<GRAD>(var, g, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
+				time = tn;
+				if (time >= end_time)
+				{
+					running = false;
+					atomicAdd(var.st.final_cnt + idx, 1u);
+					if (GRAD)
+						mbb_grad_end(g, P, discrete, C1, C2);
+					atomicAdd(var.transitions, trans);
+					trans = 0;
+				}
+				else
+				{
+					const unsigned long long r = __umul64hi(((unsigned long long)rb.y << 32) | rb.z, total);
+					unsigned long long pre = 0, cum = 0;
+					int word = 0;
+#pragma unroll
+					for (int w = 0; w < MB_LW - 1; w++)
+					{
+						pre += q[w];
+						const bool le = pre <= r;
+						word += le ? 1 : 0;
+						cum = le ? pre : cum;
+					}
+					uint32_t um = v.pick(v.u, word);
+					const uint32_t sw = v.pick(v.s, word);
+					uint32_t left = (uint32_t)(r - cum); // below the word's sum, which is below 2^32
+					j = 32 * word + 31 - __clz(um | 1u);
+					while (um)
+					{
+						const int b0 = __ffs(um) - 1;
+						const uint32_t um1 = um & (um - 1u);
+						const int b1 = um1 ? __ffs(um1) - 1 : b0;
+						const uint2 qq0 = __ldg(var.q + 32 * word + b0);
+						const uint2 qq1 = __ldg(var.q + 32 * word + b1);
+						const uint32_t qa = ((sw >> b0) & 1u) ? qq0.y : qq0.x;
+						j = 32 * word + b0;
+						if (left < qa || !um1)
+							break;
+						left -= qa;
+						const uint32_t qb = ((sw >> b1) & 1u) ? qq1.y : qq1.x;
+						j = 32 * word + b1;
+						if (left < qb)
+							break;
+						left -= qb;
+						um = um1 & (um1 - 1u);
+					}
+					if (GRAD)
+					{
+						const int jdir = (sw >> (j & 31)) & 1u; // 0: j switches on (up rate), 1: off (down rate)
+						const float rj = __ldg(var.rate + 2 * j + jdir);
+						const int a = __ldg(var.g_ptr + 2 * j + jdir), b = __ldg(var.g_ptr + 2 * j + jdir + 1);
+						for (int e = a; e < b; e++)
+						{
+							const int p = __ldg(var.g_p + e);
+							const float dA = __ldg(var.g_d + e) / rj;
+							if (!discrete)
+								mbb_red_add(g.GR(p), -(double)dA * C1);
+							g.GS(p) += dA;
+						}
+						if (discrete)
+							for (int p = 0; p < P; p++)
+								g.GS(p) -= g.GD(p) / a0;
+					}
+					mb_lock_flip(ns, v, j);
+					const int pj = (int)(__ldg(reinterpret_cast<const uint2*>(mbg_inc_dep) + j).y >> 16) - 1;
+					if (pj >= 0)
+						idx ^= 1u << pj;
+				}
+			}
+		}
+	}
+	if (acc_var >= 0)
+	{
+		mb_acc_flush(acc, B.vars[acc_var].st, B.vars[acc_var].st.win_h);
+		if (GRAD)
+			mbb_grad_emit(B.vars[acc_var], g, P);
+	}
+}
+#endif // MBG_GATES
+
 extern "C" __global__ void __launch_bounds__(128, 5) mb_batched_fast_static(mb_batch_params B)
 {
+#ifdef MBG_GATES
+	mbb_lock_body<false>(B);
+#else
 	mbb_body<false, mbb_net_static>(B);
+#endif
 }
 extern "C" __global__ void __launch_bounds__(128, 5) mb_batched_grad_static(mb_batch_params B)
 {
+#ifdef MBG_GATES
+	mbb_lock_body<true>(B);
+#else
 	mbb_body<true, mbb_net_static>(B);
+#endif
 }
 #endif
