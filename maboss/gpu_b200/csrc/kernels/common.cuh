@@ -238,14 +238,20 @@ __device__ __forceinline__ void mb_tail_add(const mb_stats_params& p, float max_
 }
 #endif
 
-// Discrete time: count the state at window lround(t0 / tick) (window_average_small.cu:117-130).
+// Discrete time: count the state at window lround(t0 / tick) (window_average_small.cu:117-130). `counts`: the
+// block's own counts in shared memory, or null.
 __device__ __forceinline__ void mb_record_disc(const mb_stats_params& p, long long* hsink, mb_idx_t idx, float t0,
-											   float h)
+											   float h, unsigned* counts = nullptr)
 {
 	const int w = (int)lroundf(t0 / p.win_tick);
 	if (w >= 0 && w < p.n_windows)
 	{
-		mb_cnt_add(p, w, idx);
+#ifndef MBG_WIDE_INDEX
+		if (counts)
+			atomicAdd(counts + (size_t)w * p.n_bins + idx, 1u);
+		else
+#endif
+			mb_cnt_add(p, w, idx);
 		mb_add_h(hsink, w, __double2ll_rn((double)h * p.fx_h));
 	}
 }

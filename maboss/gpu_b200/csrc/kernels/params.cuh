@@ -14,6 +14,11 @@ struct mb_stats_params
 	unsigned n_bins;	  // S = 2^k
 	float win_tick;		  // window size (exact host float, window_average_small.cpp:305)
 	int h_in_smem;		  // transition-entropy sums privatised per block in shared memory
+	// discrete counts privatised per block in shared memory (lockstep kernels, small histograms): all
+	// trajectories are in the same window, so their adds meet in one or two memory sectors. 10-node example
+	// model (25 windows x 16 states), 1e6 trajectories
+	// 4.2 -> 0.78 ms (0.77 without any add)
+	int cnt_in_smem;
 	double fx;			  // occupancy scale 2^e
 	double fx_h;		  // transition-entropy scale 2^eh
 	long long* win_occ;	  // [T*S] continuous occupancy (fixed point)

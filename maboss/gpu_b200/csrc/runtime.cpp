@@ -1023,6 +1023,11 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 	}
 	int block = c.block;
 	size_t smem = st.h_smem();
+	// discrete counts in shared memory: histograms of at most 16 KB, so that the occupancy stays (lockstep kernels)
+	P.st.cnt_in_smem = m.gate_words && (c.mode == MB_MODE_FUSED_EXACT || m.fast_incremental()) && st.discrete_time &&
+					   !st.wide && (size_t)st.n_windows * st.n_bins <= 4096;
+	if (P.st.cnt_in_smem)
+		smem += (size_t)st.n_windows * st.n_bins * sizeof(unsigned);
 	if (c.mode == MB_MODE_FUSED_EXACT ? m.incremental : m.fast_incremental())
 	{
 		// per thread in shared memory: state words, unstable masks and word rate sums; or per warp its array
