@@ -1069,9 +1069,21 @@ mb_status mb_result_window_probs(mb_result r, double* probs)
 			});
 			return;
 		}
-		for (int w = 0; w < x.n_windows; w++)
-			for (unsigned b = 0; b < x.n_bins; b++)
-				probs[(size_t)w * x.n_bins + b] = x.n_traj > 0 ? x.window_prob(w, b) : 0.0;
+		const size_t cells = (size_t)x.n_windows * x.n_bins;
+		if (x.n_traj <= 0)
+			std::fill_n(probs, cells, 0.0);
+		else // the divisions of result::window_prob (the one by fx, a power of two, as a product)
+		{
+			const double n = (double)x.n_traj, d = n * (double)x.time_tick, inv_fx = 1.0 / x.fx;
+			mb::parallel_ranges(cells, (int)std::thread::hardware_concurrency(), [&](size_t a, size_t e) {
+				if (x.discrete_time)
+					for (size_t i = a; i < e; i++)
+						probs[i] = (double)x.win_cnt[i] / n;
+				else
+					for (size_t i = a; i < e; i++)
+						probs[i] = ((double)x.win_occ[i] * inv_fx) / d;
+			});
+		}
 	});
 }
 

@@ -216,14 +216,96 @@ dbuf::~dbuf()
 		cudaFree(p);
 }
 
-void host_deleter::operator()(void* p) const
+namespace {
+// returned blocks of host_stage, the longest unused first (never destroyed: the driver may be gone at
+// process exit)
+struct stage_pool
+{
+	std::mutex mu;
+	std::vector<std::pair<size_t, void*>> blocks;
+	size_t kept = 0;
+	static constexpr size_t most = 64ull << 20;
+};
+stage_pool& stages()
+{
+	static stage_pool* pool = new stage_pool;
+	return *pool;
+}
+} // namespace
+
+void host_stage::reserve(size_t bytes)
+{
+	if (bytes <= size)
+		return;
+	release();
+	size_t want = 4096;
+	while (want < bytes)
+		want <<= 1;
+	stage_pool& pool = stages();
+	{
+		std::lock_guard<std::mutex> lk(pool.mu);
+		for (size_t i = pool.blocks.size(); i-- > 0;)
+			if (pool.blocks[i].first == want)
+			{
+				p = pool.blocks[i].second;
+				pool.blocks.erase(pool.blocks.begin() + (std::ptrdiff_t)i);
+				pool.kept -= want;
+				size = want;
+				pinned = true;
+				return;
+			}
+	}
+	pinned = cudaHostAlloc(&p, want, cudaHostAllocPortable) == cudaSuccess;
+	if (!pinned)
+	{
+		(void)cudaGetLastError();
+		p = std::malloc(want);
+		if (!p)
+			throw engine_error(MB_ERR_LIMIT, "out of host memory for the result's copies");
+	}
+	size = want;
+}
+
+void host_stage::release() noexcept
 {
 	if (!p)
 		return;
-	if (pinned)
-		cudaFreeHost(p);
-	else
+	std::vector<void*> freed;
+	if (!pinned)
 		std::free(p);
+	else
+	{
+		stage_pool& pool = stages();
+		bool keep = size <= stage_pool::most;
+		{
+			std::lock_guard<std::mutex> lk(pool.mu);
+			try
+			{
+				if (keep)
+				{
+					freed.reserve(pool.blocks.size());
+					pool.blocks.emplace_back(size, p);
+					pool.kept += size;
+				}
+			}
+			catch (...)
+			{
+				keep = false;
+			}
+			while (pool.kept > stage_pool::most) // (the block just returned is the last, and fits alone)
+			{
+				freed.push_back(pool.blocks.front().second);
+				pool.kept -= pool.blocks.front().first;
+				pool.blocks.erase(pool.blocks.begin());
+			}
+		}
+		if (!keep)
+			cudaFreeHost(p);
+		for (void* q : freed)
+			cudaFreeHost(q);
+	}
+	p = nullptr;
+	size = 0;
 }
 
 void dbuf::alloc(size_t n)
@@ -270,6 +352,9 @@ module::~module()
 {
 	cudaSetDevice(ctx->device);
 	last_runner.reset();
+	for (cudaEvent_t e : { run0, run1 })
+		if (e)
+			cudaEventDestroy(e);
 	for (int f = 0; f < FAMILY_COUNT; f++)
 		if (mods[f] && f != FAMILY_BATCH)
 			drv().ModuleUnload(mods[f]);
@@ -565,35 +650,6 @@ void stats_state::init(module& m, float tick, float tmax, bool discrete, const s
 										: std::max(1u << 16, (unsigned)std::min<unsigned long long>(next_pow2(4 * want), 1ull << 28));
 		bin_keys.alloc((size_t)bin_cap * sizeof(mb_key128));
 		bin_vals.alloc((size_t)bin_cap * sizeof(long long));
-		MB_CUDA(cudaMemsetAsync(bin_keys.p, 0, bin_keys.bytes, s));
-		MB_CUDA(cudaMemsetAsync(bin_vals.p, 0, bin_vals.bytes, s));
-	}
-	if ((sections & 1u) && wide)
-	{
-		h.alloc(n_windows * sizeof(long long));
-		MB_CUDA(cudaMemsetAsync(h.p, 0, h.bytes, s));
-	}
-	else if (sections & 1u)
-	{
-		if (discrete)
-		{
-			cnt.alloc(cells * sizeof(unsigned));
-			MB_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes, s));
-		}
-		else
-		{
-			// the counts of trajectories at a fixed point behind the sums: one clear for both
-			has_tail = cells <= tail_max_cells;
-			occ.alloc(cells * (sizeof(long long) + (has_tail ? sizeof(unsigned) : 0)));
-			MB_CUDA(cudaMemsetAsync(occ.p, 0, occ.bytes, s));
-		}
-		h.alloc(n_windows * sizeof(long long));
-		MB_CUDA(cudaMemsetAsync(h.p, 0, h.bytes, s));
-	}
-	if ((sections & 2u) && !wide)
-	{
-		fin.alloc(n_bins * sizeof(unsigned));
-		MB_CUDA(cudaMemsetAsync(fin.p, 0, fin.bytes, s));
 	}
 	fp_cap = 0;
 	if (sections & 4u)
@@ -601,14 +657,33 @@ void stats_state::init(module& m, float tick, float tmax, bool discrete, const s
 		fp_cap = fixed_capacity_log2 > 0
 					 ? (1u << std::min(fixed_capacity_log2, 28))
 					 : next_pow2((unsigned long long)std::max(1024LL, std::min(std::max(n, 0LL), 1LL << 22) * 2));
-		fp_keys.alloc((size_t)fp_cap * sizeof(mb_key128));
-		fp_counts.alloc((size_t)fp_cap * sizeof(unsigned));
 		fp_states.alloc((size_t)fp_cap * m.state_words * sizeof(unsigned));
-		MB_CUDA(cudaMemsetAsync(fp_keys.p, 0, fp_keys.bytes, s));
-		MB_CUDA(cudaMemsetAsync(fp_counts.p, 0, fp_counts.bytes, s));
 	}
-	counters.alloc(64);
-	MB_CUDA(cudaMemsetAsync(counters.p, 0, 64, s));
+	// the counts of trajectories at a fixed point are behind the occupancy sums
+	has_tail = (sections & 1u) && !wide && !discrete && cells <= tail_max_cells;
+	const std::pair<dview*, size_t> parts[] = {
+		{ &counters, 64 },
+		{ &h, (sections & 1u) ? n_windows * sizeof(long long) : 0 },
+		{ &fin, (sections & 2u) && !wide ? n_bins * sizeof(unsigned) : 0 },
+		{ &cnt, (sections & 1u) && !wide && discrete ? cells * sizeof(unsigned) : 0 },
+		{ &occ, (sections & 1u) && !wide && !discrete
+					? cells * (sizeof(long long) + (has_tail ? sizeof(unsigned) : 0))
+					: 0 },
+		{ &fp_keys, (size_t)fp_cap * sizeof(mb_key128) },
+		{ &fp_counts, (size_t)fp_cap * sizeof(unsigned) },
+	};
+	size_t total = 0;
+	for (const auto& part : parts)
+		total += (part.second + 255) / 256 * 256;
+	arena.alloc(total);
+	size_t at = 0;
+	for (const auto& part : parts)
+	{
+		part.first->bytes = part.second;
+		part.first->p = part.second ? static_cast<char*>(arena.p) + at : nullptr;
+		at += (part.second + 255) / 256 * 256;
+	}
+	zero(s);
 
 	p = mb_stats_params{};
 	p.n_windows = n_windows;
@@ -635,9 +710,10 @@ void stats_state::init(module& m, float tick, float tmax, bool discrete, const s
 
 void stats_state::zero(cudaStream_t s)
 {
-	for (dbuf* b : { &occ, &cnt, &h, &fin, &fp_keys, &fp_counts, &counters, &bin_keys, &bin_vals })
+	for (dbuf* b : { &arena, &bin_keys, &bin_vals })
 		if (b->p)
 			MB_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, s));
+	extracted = false;
 }
 
 void stats_state::set_istate(const std::vector<float>& is, cudaStream_t s)
@@ -706,7 +782,12 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 	const size_t cells = (size_t)n_windows * n_bins;
 	// compact the occupied fixed-point slots on the device; the same launch adds the window sums of the
 	// trajectories that were counted at their fixed point (and clears the counts)
-	MB_CUDA(cudaMemsetAsync(extract_ctr(), 0, sizeof(unsigned), s));
+	if (extracted)
+	{
+		MB_CUDA(cudaMemsetAsync(extract_ctr(), 0, sizeof(unsigned), s));
+		MB_CUDA(cudaMemsetAsync(bin_extract_ctr(), 0, sizeof(unsigned), s));
+	}
+	extracted = true;
 	// compaction buffers, allocated with the first result and kept for the next runs
 	if (fp_cap && out_counts.bytes != (size_t)fp_cap * sizeof(unsigned))
 	{
@@ -736,7 +817,6 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 			out_bin_keys.alloc((size_t)bin_cap * sizeof(mb_key128));
 			out_bin_vals.alloc((size_t)bin_cap * sizeof(long long));
 		}
-		MB_CUDA(cudaMemsetAsync(bin_extract_ctr(), 0, sizeof(unsigned), s));
 		unsigned cap = bin_cap;
 		mb_key128* keys = p.bin_keys;
 		long long* vals = p.bin_vals;
@@ -749,45 +829,20 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 		MB_CUDA(cudaMemcpyAsync(&nb, bin_extract_ctr(), sizeof nb, cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaMemcpyAsync(&ovf, bin_overflow_ctr(), sizeof ovf, cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaStreamSynchronize(s));
-		// sorted on the device, copied into the kept host buffers, decoded by host threads
-		if (nb > hbin_cap)
-		{
-			hbin_keys.reset();
-			hbin_vals.reset();
-			hbin_cap = 0;
-			auto host_alloc = [](size_t bytes, bool& pinned) {
-				void* p = nullptr;
-				pinned = cudaMallocHost(&p, bytes) == cudaSuccess;
-				if (!pinned)
-				{
-					(void)cudaGetLastError();
-					p = std::malloc(bytes);
-					if (!p)
-						throw engine_error(MB_ERR_LIMIT, "out of host memory for the sparse bins");
-				}
-				return p;
-			};
-			void* hk = host_alloc(2 * (size_t)nb * sizeof(uint64_t), hbin_keys.get_deleter().pinned);
-			hbin_keys.reset(static_cast<uint64_t*>(hk));
-			void* hv = host_alloc((size_t)nb * sizeof(long long), hbin_vals.get_deleter().pinned);
-			hbin_vals.reset(static_cast<long long*>(hv));
-			hbin_cap = nb;
-		}
+		// sorted on the device, copied into pinned memory, decoded by host threads
+		stage_keys.reserve((size_t)nb * sizeof(mb_key128));
+		stage_vals.reserve((size_t)nb * sizeof(long long));
 		if (nb)
 		{
-			dbuf sk((size_t)nb * sizeof(mb_key128)), sv((size_t)nb * sizeof(long long));
-			sort_bins(ok, ov, nb, sk.as<mb_key128>(), sv.as<long long>(), s);
-			MB_CUDA(cudaMemcpy(hbin_keys.get(), sk.p, nb * sizeof(mb_key128), cudaMemcpyDeviceToHost));
-			MB_CUDA(cudaMemcpy(hbin_vals.get(), sv.p, nb * sizeof(long long), cudaMemcpyDeviceToHost));
+			sort_bins(ok, ov, nb, scratch, s);
+			MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), scratch.out_keys.p, nb * sizeof(mb_key128), cudaMemcpyDeviceToHost, s));
+			MB_CUDA(cudaMemcpyAsync(stage_vals.as<void>(), scratch.out_vals.p, nb * sizeof(long long), cudaMemcpyDeviceToHost, s));
+			MB_CUDA(cudaStreamSynchronize(s));
 		}
-		decode_sorted_bins(hbin_keys.get(), hbin_vals.get(), nb, n_windows, (int)std::thread::hardware_concurrency(),
+		decode_sorted_bins(stage_keys.as<uint64_t>(), stage_vals.as<long long>(), nb, n_windows, (int)std::thread::hardware_concurrency(),
 						   r.sp_w, r.sp_idx, r.sp_val, r.sp_begin, r.fin_idx, r.fin_cnt);
+		scratch.trim();
 		r.bin_overflow = ovf;
-	}
-	if ((sections & 1u) && wide)
-	{
-		r.win_h.resize(n_windows);
-		MB_CUDA(cudaMemcpyAsync(r.win_h.data(), h.p, n_windows * sizeof(long long), cudaMemcpyDeviceToHost, s));
 	}
 	// a large dense histogram: only its non-zero cells (selected on the device in cell order), when
 	// they are at most a quarter of it
@@ -795,26 +850,30 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 	{
 		const long long nz = compact_cells(discrete_time ? nullptr : occ.as<long long>(),
 										   discrete_time ? cnt.as<unsigned>() : nullptr, cells, cells / 4, cell_idx,
-										   cell_vals, m.ctx->sm_count, s);
+										   cell_vals, m.ctx->sm_count, scratch, s);
 		if (nz >= 0)
 		{
-			std::vector<unsigned long long> idx((size_t)nz);
-			r.sp_val.resize((size_t)nz);
+			stage_keys.reserve((size_t)nz * sizeof(unsigned long long));
+			stage_vals.reserve((size_t)nz * sizeof(long long));
 			if (nz)
 			{
-				MB_CUDA(cudaMemcpyAsync(idx.data(), cell_idx.p, (size_t)nz * sizeof(unsigned long long),
+				MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), cell_idx.p, (size_t)nz * sizeof(unsigned long long),
 										cudaMemcpyDeviceToHost, s));
-				MB_CUDA(cudaMemcpyAsync(r.sp_val.data(), cell_vals.p, (size_t)nz * sizeof(long long),
+				MB_CUDA(cudaMemcpyAsync(stage_vals.as<void>(), cell_vals.p, (size_t)nz * sizeof(long long),
 										cudaMemcpyDeviceToHost, s));
 				MB_CUDA(cudaStreamSynchronize(s));
 			}
+			const unsigned long long* idx = stage_keys.as<unsigned long long>();
+			const long long* vals = stage_vals.as<long long>();
 			r.sp_w.resize((size_t)nz);
 			r.sp_idx.resize((size_t)nz);
+			r.sp_val.resize((size_t)nz);
 			parallel_ranges((size_t)nz, (int)std::thread::hardware_concurrency(), [&](size_t a, size_t e) {
 				for (size_t i = a; i < e; i++)
 				{
 					r.sp_w[i] = (int)(idx[i] / n_bins);
 					r.sp_idx[i] = (unsigned __int128)(idx[i] % n_bins);
+					r.sp_val[i] = vals[i];
 				}
 			});
 			r.sp_begin.assign((size_t)n_windows + 1, 0);
@@ -823,43 +882,68 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 			r.compact = true;
 		}
 	}
-	if ((sections & 1u) && !wide && !r.compact && discrete_time)
+	// counters, entropy sums, final states and a window histogram of at most 32 MB in one copy, with the first
+	// fixed points; a larger histogram straight into the result
+	const dview& win = discrete_time ? cnt : occ;
+	const size_t win_bytes = cells * (discrete_time ? sizeof(unsigned) : sizeof(long long));
+	const bool has_win = (sections & 1u) && !wide && !r.compact, win_staged = has_win && win_bytes <= (32u << 20);
+	auto offset = [&](const dview& v) { return (size_t)(static_cast<char*>(v.p) - static_cast<char*>(arena.p)); };
+	size_t front = 64;
+	if (h.p)
+		front = offset(h) + h.bytes;
+	if (fin.p)
+		front = offset(fin) + fin.bytes;
+	if (win_staged)
+		front = offset(win) + win_bytes;
+	front = (front + 255) / 256 * 256;
+	const int W = m.state_words;
+	const unsigned first = std::min(fp_cap, 256u); // fixed points copied before their number is known
+	stage.reserve(front + (size_t)first * (W + 1) * sizeof(unsigned));
+	const size_t at_counts = front, at_states = front + first * sizeof(unsigned);
+	MB_CUDA(cudaMemcpyAsync(stage.as<void>(), arena.p, std::min(front, arena.bytes), cudaMemcpyDeviceToHost, s));
+	if (first)
 	{
-		r.win_cnt.resize(cells);
-		MB_CUDA(cudaMemcpyAsync(r.win_cnt.data(), cnt.p, cells * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		MB_CUDA(cudaMemcpyAsync(stage.as<void>(at_counts), out_counts.p, first * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		MB_CUDA(cudaMemcpyAsync(stage.as<void>(at_states), out_states.p, (size_t)first * W * sizeof(unsigned),
+								cudaMemcpyDeviceToHost, s));
 	}
-	else if ((sections & 1u) && !wide && !r.compact)
+	if (has_win && !win_staged)
 	{
-		r.win_occ.resize(cells);
-		MB_CUDA(cudaMemcpyAsync(r.win_occ.data(), occ.p, cells * sizeof(long long), cudaMemcpyDeviceToHost, s));
+		if (discrete_time)
+			r.win_cnt.resize(cells);
+		else
+			r.win_occ.resize(cells);
+		void* to = discrete_time ? static_cast<void*>(r.win_cnt.data()) : static_cast<void*>(r.win_occ.data());
+		MB_CUDA(cudaMemcpyAsync(to, win.p, win_bytes, cudaMemcpyDeviceToHost, s));
 	}
-	if (sections & 1u)
-	{
-		r.win_h.resize(n_windows);
-		MB_CUDA(cudaMemcpyAsync(r.win_h.data(), h.p, n_windows * sizeof(long long), cudaMemcpyDeviceToHost, s));
-	}
-	if ((sections & 2u) && !wide)
-	{
-		r.final_cnt.resize(n_bins);
-		MB_CUDA(cudaMemcpyAsync(r.final_cnt.data(), fin.p, n_bins * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-	}
-
-	unsigned ctr[8];
-	unsigned long long trans = 0;
-	MB_CUDA(cudaMemcpyAsync(ctr, counters.p, sizeof ctr, cudaMemcpyDeviceToHost, s));
-	MB_CUDA(cudaMemcpyAsync(&trans, transitions(), sizeof trans, cudaMemcpyDeviceToHost, s));
 	MB_CUDA(cudaStreamSynchronize(s));
-	r.transitions = trans;
+	const unsigned* ctr = stage.as<unsigned>();
+	std::memcpy(&r.transitions, stage.as<char>(sizeof(unsigned long long)), sizeof r.transitions);
 	r.fixed_overflow = ctr[4];
 	r.rate_errors = ctr[6];
 	const unsigned nfp = ctr[5];
-	const int W = m.state_words;
+	if (h.p)
+		r.win_h.assign(stage.as<long long>(offset(h)), stage.as<long long>(offset(h)) + n_windows);
+	if (fin.p)
+		r.final_cnt.assign(stage.as<unsigned>(offset(fin)), stage.as<unsigned>(offset(fin)) + n_bins);
+	if (win_staged && discrete_time)
+		r.win_cnt.assign(stage.as<unsigned>(offset(cnt)), stage.as<unsigned>(offset(cnt)) + cells);
+	else if (win_staged)
+		r.win_occ.assign(stage.as<long long>(offset(occ)), stage.as<long long>(offset(occ)) + cells);
 	std::vector<unsigned> st((size_t)nfp * W), cn(nfp);
-	if (nfp)
+	if (nfp > first)
 	{
-		MB_CUDA(cudaMemcpyAsync(st.data(), out_states.p, st.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(cn.data(), out_counts.p, cn.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		stage_keys.reserve((size_t)nfp * (W + 1) * sizeof(unsigned));
+		MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), out_counts.p, nfp * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		MB_CUDA(cudaMemcpyAsync(stage_keys.as<unsigned>() + nfp, out_states.p, st.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaStreamSynchronize(s));
+		std::copy_n(stage_keys.as<unsigned>(), nfp, cn.begin());
+		std::copy_n(stage_keys.as<unsigned>() + nfp, st.size(), st.begin());
+	}
+	else
+	{
+		std::copy_n(stage.as<unsigned>(at_counts), nfp, cn.begin());
+		std::copy_n(stage.as<unsigned>(at_states), st.size(), st.begin());
 	}
 	set_fixed_sorted(r, st, cn);
 	return rp;
@@ -1255,10 +1339,9 @@ runner::runner(module& m, const run_config& c) : mod(&m), cfg(c)
 runner::~runner()
 {
 	cudaSetDevice(mod->ctx->device);
-	if (ev0)
-		cudaEventDestroy(ev0);
-	if (ev1)
-		cudaEventDestroy(ev1);
+	for (cudaEvent_t e : { ev0, ev1 })
+		if (e)
+			cudaEventDestroy(e);
 }
 
 unsigned runner::kernel_launches() const { return launches; }
@@ -1364,27 +1447,23 @@ std::unique_ptr<result> run(module& m, const run_config& c)
 	// the module keeps the runner (device buffers) of its last run and reuses it for the same config
 	std::lock_guard<std::mutex> lk(m.run_mu);
 	cudaStream_t s = m.ctx->stream;
-	cudaEvent_t t0, t1;
 	MB_CUDA(cudaSetDevice(m.ctx->device));
-	MB_CUDA(cudaEventCreate(&t0));
-	MB_CUDA(cudaEventCreate(&t1));
-	MB_CUDA(cudaEventRecord(t0, s));
-	std::unique_ptr<result> r;
+	if (!m.run0)
+		MB_CUDA(cudaEventCreate(&m.run0));
+	if (!m.run1)
+		MB_CUDA(cudaEventCreate(&m.run1));
+	MB_CUDA(cudaEventRecord(m.run0, s));
+	if (!m.last_runner || !same_run(m.last_runner->cfg, c))
 	{
-		if (!m.last_runner || !same_run(m.last_runner->cfg, c))
-		{
-			m.last_runner.reset();
-			m.last_runner = std::make_unique<runner>(m, c);
-		}
-		runner& rn = *m.last_runner;
-		rn.launch(s);
-		r = rn.collect(s);
+		m.last_runner.reset();
+		m.last_runner = std::make_unique<runner>(m, c);
 	}
-	MB_CUDA(cudaEventRecord(t1, s));
-	MB_CUDA(cudaEventSynchronize(t1));
-	MB_CUDA(cudaEventElapsedTime(&r->total_ms, t0, t1));
-	cudaEventDestroy(t0);
-	cudaEventDestroy(t1);
+	runner& rn = *m.last_runner;
+	rn.launch(s);
+	std::unique_ptr<result> r = rn.collect(s);
+	MB_CUDA(cudaEventRecord(m.run1, s));
+	MB_CUDA(cudaEventSynchronize(m.run1));
+	MB_CUDA(cudaEventElapsedTime(&r->total_ms, m.run0, m.run1));
 	return r;
 }
 

@@ -81,6 +81,63 @@ struct dbuf
 	}
 };
 
+// A part of a dbuf.
+struct dview
+{
+	void* p = nullptr;
+	size_t bytes = 0;
+	template <typename T>
+	T* as() const
+	{
+		return static_cast<T*>(p);
+	}
+};
+
+// Pinned host memory for the copies of a result. Allocating it takes 0.7 ms a MB, so a run's statistics keep
+// theirs, and it comes from and goes back to a pool of the process: blocks of power-of-two sizes, at most
+// 64 MB of them, the longest unused freed first. Any thread may borrow and return. Where pinning fails,
+// plain memory.
+class host_stage
+{
+public:
+	host_stage() = default;
+	~host_stage() { release(); }
+	host_stage(const host_stage&) = delete;
+	host_stage& operator=(const host_stage&) = delete;
+	void reserve(size_t bytes); // (what it held is lost)
+	template <typename T>
+	T* as(size_t offset = 0) const
+	{
+		return reinterpret_cast<T*>(static_cast<char*>(p) + offset);
+	}
+
+private:
+	void release() noexcept;
+	void* p = nullptr;
+	size_t size = 0;
+	bool pinned = true;
+};
+
+// Device scratch of sort_bins and compact_cells, kept between runs.
+struct sort_scratch
+{
+	dbuf lo, lo_sorted, hi, hi_sorted, pos, pos_a, pos_b, tmp, counters, out_keys, out_vals;
+	static void reserve(dbuf& b, size_t bytes)
+	{
+		if (b.bytes < bytes)
+			b.alloc(bytes + bytes / 4);
+	}
+	// gives back more than 1 GB (its work has been waited for)
+	void trim()
+	{
+		size_t total = 0;
+		for (const dbuf* b : { &lo, &lo_sorted, &hi, &hi_sorted, &pos, &pos_a, &pos_b, &tmp, &out_keys, &out_vals })
+			total += b->bytes;
+		if (total > (1ull << 30))
+			*this = sort_scratch();
+	}
+};
+
 struct context
 {
 	int device = 0;
@@ -131,6 +188,7 @@ struct module
 	std::string source; // generated model source that was compiled with the engine
 	std::mutex run_mu;	// whole runs (run()) of this module are serialised
 	std::unique_ptr<struct runner> last_runner; // buffers of the last run(), reused for the same config
+	cudaEvent_t run0 = nullptr, run1 = nullptr; // around a whole run()
 	std::string log;	// NVRTC log
 
 	CUfunction fused_exact = nullptr, fused_fast = nullptr;
@@ -168,10 +226,11 @@ void simulate_epoch(module& m, bool dense, cudaStream_t s, int n, int stride, in
 // val_out (int64), both grown as needed. Returns the number of cells, or -1 without writing them
 // when there are more than max_entries (the dense copy is then cheaper).
 long long compact_cells(const long long* occ, const unsigned* cnt, unsigned long long cells,
-						unsigned long long max_entries, dbuf& idx_out, dbuf& val_out, int sm_count, cudaStream_t s);
+						unsigned long long max_entries, dbuf& idx_out, dbuf& val_out, int sm_count,
+						sort_scratch& scratch, cudaStream_t s);
 
-void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, mb_key128* out_keys, long long* out_vals,
-			   cudaStream_t s);
+// (asynchronous; the sorted bins are in scratch.out_keys and scratch.out_vals)
+void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, sort_scratch& scratch, cudaStream_t s);
 
 // Stable partition of the CONTINUE trajectories of an epoch batch into another buffer set
 // (last_states SoA [word * stride + i], last_times, random states); the number kept is written to
@@ -268,28 +327,23 @@ std::unique_ptr<result> merge_results(const std::vector<const result*>& parts);
 int occupancy_exponent(long long n_traj, float tick, bool discrete);
 int entropy_exponent(long long n_traj, float tick, bool discrete);
 
-// Frees host memory from cudaMallocHost (pinned) or, where pinning failed, from malloc.
-struct host_deleter
-{
-	bool pinned = true;
-	void operator()(void* p) const;
-};
-
 // Device accumulators of the three built-in statistics plugins (window averages, final
 // states, fixed points) for one run.
 struct stats_state
 {
 	module* mod = nullptr;
-	dbuf occ, cnt, h, fin, fp_keys, fp_counts, fp_states, counters, istate;
+	// one buffer for all accumulators that a launch clears (one clear), in the order counters, h, fin, occ or
+	// cnt, fp_keys, fp_counts: the part that a result copies back is at its front (one copy)
+	dbuf arena;
+	dview occ, cnt, h, fin, fp_keys, fp_counts, counters;
+	dbuf fp_states, istate;
+	bool extracted = false; // the extraction counters are not cleared since the last finalize
 	dbuf out_counts, out_states; // compacted fixed points (finalize)
 	dbuf bin_keys, bin_vals, out_bin_keys, out_bin_vals; // sparse bins (more than 20 non-internal nodes)
 	dbuf cell_idx, cell_vals; // non-zero cells of a large dense histogram (compact results), kept across runs
+	sort_scratch scratch;
+	host_stage stage, stage_keys, stage_vals; // a result's copies, kept across runs
 	unsigned bin_cap = 0;
-	// host copies of the sorted bins, kept across runs (no re-allocation, no first-touch page
-	// faults), in pinned memory (copied at full link speed) unless pinning fails (then malloc)
-	std::unique_ptr<uint64_t[], host_deleter> hbin_keys;
-	std::unique_ptr<long long[], host_deleter> hbin_vals;
-	size_t hbin_cap = 0;
 	bool wide = false;
 	bool has_tail = false; // occ is followed by the counts of mb_record_fixed (u32 per cell)
 	unsigned fp_cap = 0;

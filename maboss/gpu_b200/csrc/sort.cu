@@ -48,13 +48,17 @@ __global__ void mbs_gather(unsigned n, const mb_key128* __restrict__ keys, const
 
 } // namespace
 
-void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, mb_key128* out_keys, long long* out_vals,
-			   cudaStream_t s)
+void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, sort_scratch& x, cudaStream_t s)
 {
 	if (n == 0)
 		return;
-	dbuf lo((size_t)n * 8), lo_sorted((size_t)n * 8), hi((size_t)n * 8), hi_sorted((size_t)n * 8);
-	dbuf pos((size_t)n * 4), pos_a((size_t)n * 4), pos_b((size_t)n * 4);
+	for (dbuf* b : { &x.lo, &x.lo_sorted, &x.hi, &x.hi_sorted, &x.out_vals })
+		sort_scratch::reserve(*b, (size_t)n * 8);
+	for (dbuf* b : { &x.pos, &x.pos_a, &x.pos_b })
+		sort_scratch::reserve(*b, (size_t)n * 4);
+	sort_scratch::reserve(x.out_keys, (size_t)n * sizeof(mb_key128));
+	dbuf &lo = x.lo, &lo_sorted = x.lo_sorted, &hi = x.hi, &hi_sorted = x.hi_sorted;
+	dbuf &pos = x.pos, &pos_a = x.pos_a, &pos_b = x.pos_b, &tmp = x.tmp;
 	const unsigned grid = (n + 255) / 256;
 	mbs_split<<<grid, 256, 0, s>>>(n, keys, lo.as<unsigned long long>(), pos.as<unsigned>());
 	MB_CUDA(cudaGetLastError());
@@ -65,20 +69,19 @@ void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, mb_key1
 	MB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp2, hi.as<unsigned long long>(),
 											hi_sorted.as<unsigned long long>(), pos_a.as<unsigned>(),
 											pos_b.as<unsigned>(), (int)n, 0, 64, s));
-	dbuf tmp(std::max(tmp_bytes, tmp2));
+	sort_scratch::reserve(tmp, std::max(tmp_bytes, tmp2));
 	// by the low word, then (stable) by the high word
 	MB_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, lo.as<unsigned long long>(),
 											lo_sorted.as<unsigned long long>(), pos.as<unsigned>(),
 											pos_a.as<unsigned>(), (int)n, 0, 64, s));
 	mbs_gather_hi<<<grid, 256, 0, s>>>(n, keys, pos_a.as<unsigned>(), hi.as<unsigned long long>());
 	MB_CUDA(cudaGetLastError());
-	tmp2 = tmp.bytes;
 	MB_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tmp2, hi.as<unsigned long long>(),
 											hi_sorted.as<unsigned long long>(), pos_a.as<unsigned>(),
 											pos_b.as<unsigned>(), (int)n, 0, 64, s));
-	mbs_gather<<<grid, 256, 0, s>>>(n, keys, vals, pos_b.as<unsigned>(), out_keys, out_vals);
+	mbs_gather<<<grid, 256, 0, s>>>(n, keys, vals, pos_b.as<unsigned>(), x.out_keys.as<mb_key128>(),
+									x.out_vals.as<long long>());
 	MB_CUDA(cudaGetLastError());
-	MB_CUDA(cudaStreamSynchronize(s)); // the scratch buffers are released on return
 }
 
 namespace {
@@ -116,12 +119,12 @@ __global__ void mbs_gather_cells(unsigned long long n, const T* __restrict__ v, 
 
 template <typename T>
 long long compact_cells_t(const T* v, unsigned long long cells, unsigned long long max_entries, dbuf& idx_out,
-						  dbuf& val_out, int sm_count, cudaStream_t s)
+						  dbuf& val_out, int sm_count, sort_scratch& x, cudaStream_t s)
 {
 	if (cells == 0)
 		return 0;
-	dbuf counters(2 * sizeof(unsigned long long));
-	unsigned long long* count = counters.as<unsigned long long>();
+	sort_scratch::reserve(x.counters, 2 * sizeof(unsigned long long));
+	unsigned long long* count = x.counters.as<unsigned long long>();
 	MB_CUDA(cudaMemsetAsync(count, 0, 2 * sizeof(unsigned long long), s));
 	const unsigned grid = (unsigned)std::min<unsigned long long>((cells + 255) / 256, (unsigned long long)sm_count * 8);
 	mbs_count_nonzero<T><<<grid, 256, 0, s>>>(v, cells, count);
@@ -131,24 +134,21 @@ long long compact_cells_t(const T* v, unsigned long long cells, unsigned long lo
 	MB_CUDA(cudaStreamSynchronize(s));
 	if (n > max_entries)
 		return -1;
-	if (idx_out.bytes < n * sizeof(unsigned long long) || idx_out.bytes == 0)
-		idx_out.alloc(std::max<unsigned long long>(n, 1) * sizeof(unsigned long long));
-	if (val_out.bytes < n * sizeof(long long) || val_out.bytes == 0)
-		val_out.alloc(std::max<unsigned long long>(n, 1) * sizeof(long long));
+	sort_scratch::reserve(idx_out, std::max<unsigned long long>(n, 1) * sizeof(unsigned long long));
+	sort_scratch::reserve(val_out, std::max<unsigned long long>(n, 1) * sizeof(long long));
 	unsigned long long* idx = idx_out.as<unsigned long long>();
 	unsigned long long* selected = count + 1;
 	// in index order (window, then state): chunks of at most 2^30 cells for CUB's item count
 	const unsigned long long chunk = 1ull << 30;
 	unsigned long long written = 0;
-	dbuf tmp;
+	dbuf& tmp = x.tmp;
 	for (unsigned long long base = 0; base < cells; base += chunk)
 	{
 		const int items = (int)std::min(chunk, cells - base);
 		thrust::counting_iterator<unsigned long long> in(base);
 		size_t tmp_bytes = 0;
 		MB_CUDA(cub::DeviceSelect::If(nullptr, tmp_bytes, in, idx + written, selected, items, mbs_nonzero<T> { v }, s));
-		if (tmp.bytes < tmp_bytes)
-			tmp.alloc(tmp_bytes);
+		sort_scratch::reserve(tmp, tmp_bytes);
 		MB_CUDA(cub::DeviceSelect::If(tmp.p, tmp_bytes, in, idx + written, selected, items, mbs_nonzero<T> { v }, s));
 		unsigned long long got = 0;
 		MB_CUDA(cudaMemcpyAsync(&got, selected, sizeof got, cudaMemcpyDeviceToHost, s));
@@ -162,17 +162,17 @@ long long compact_cells_t(const T* v, unsigned long long cells, unsigned long lo
 		mbs_gather_cells<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, v, idx, val_out.as<long long>());
 		MB_CUDA(cudaGetLastError());
 	}
-	MB_CUDA(cudaStreamSynchronize(s)); // the counters and CUB scratch are released on return
 	return (long long)n;
 }
 
 } // namespace
 
 long long compact_cells(const long long* occ, const unsigned* cnt, unsigned long long cells,
-						unsigned long long max_entries, dbuf& idx_out, dbuf& val_out, int sm_count, cudaStream_t s)
+						unsigned long long max_entries, dbuf& idx_out, dbuf& val_out, int sm_count,
+						sort_scratch& scratch, cudaStream_t s)
 {
-	return occ ? compact_cells_t<long long>(occ, cells, max_entries, idx_out, val_out, sm_count, s)
-			   : compact_cells_t<unsigned>(cnt, cells, max_entries, idx_out, val_out, sm_count, s);
+	return occ ? compact_cells_t<long long>(occ, cells, max_entries, idx_out, val_out, sm_count, scratch, s)
+			   : compact_cells_t<unsigned>(cnt, cells, max_entries, idx_out, val_out, sm_count, scratch, s);
 }
 
 } // namespace mb

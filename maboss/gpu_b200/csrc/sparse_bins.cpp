@@ -77,7 +77,7 @@ void decode_sorted_bins(const uint64_t* keys, const long long* vals, size_t n, i
 						std::vector<unsigned __int128>& fin_idx, std::vector<unsigned>& fin_cnt)
 {
 	// small inputs stay on the calling thread
-	const int T = n < ((size_t)1 << 16) ? 1 : std::max(1, std::min(threads, 64));
+	const int T = std::max(1, (int)std::min<size_t>(n >> 16, (size_t)std::max(0, std::min(threads, 64))));
 	// chunk t covers [start[t], start[t + 1]); a chunk never starts inside a run of equal keys
 	std::vector<size_t> start(T + 1, n);
 	start[0] = 0;
@@ -143,7 +143,8 @@ void decode_sorted_bins(const uint64_t* keys, const long long* vals, size_t n, i
 
 void parallel_ranges(size_t n, int threads, const std::function<void(size_t, size_t)>& f)
 {
-	const int T = n < ((size_t)1 << 16) ? 1 : std::max(1, std::min(threads, 64));
+	// (a thread for every 2^16 elements at most: starting one takes as long as some thousands of them)
+	const int T = std::max(1, (int)std::min<size_t>(n >> 16, (size_t)std::max(0, std::min(threads, 64))));
 	parallel(T, [&](int t) { f(n * (size_t)t / (size_t)T, n * (size_t)(t + 1) / (size_t)T); });
 }
 

@@ -506,7 +506,7 @@ class Result:
 
     @property
     def window_probs(self) -> np.ndarray:
-        out = np.zeros((self.dims.windows, self.dims.bins), np.float64)
+        out = np.empty((self.dims.windows, self.dims.bins), np.float64)  # (every value is written)
         check(lib().mb_result_window_probs(self._h, out.ctypes.data))
         return out
 
