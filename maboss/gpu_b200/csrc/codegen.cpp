@@ -336,6 +336,7 @@ void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 	}
 	emit_array(ss, "unsigned", "mbg_inc_dep", dep2);
 	// 16-byte dependent records (the node's rates come from mbg_inc_q); inputs 4-11 apart
+	ss << "constexpr int mbg_inc_records = " << t.crec.size() / 4 << ";" << std::endl;
 	emit_array(ss, "uint4", "mbg_inc_crec", u4(t.crec));
 	emit_array(ss, "uint4", "mbg_inc_cext", u4(t.cext));
 	if (many)
@@ -424,13 +425,14 @@ void emit_incremental_tables(std::ostream& ss, const model_layout& L)
 // Tables of the lockstep kernels: the network's gates (gates.h) as {byte offset of a | of b << 16 | or <<
 // 31, byte offset of c | of d << 16 | invert << 31}, and, for models whose positive rates take at most
 // three values, the unstable nodes of each value as masks (their sums are then population counts).
-void emit_gates(std::ostream& ss, const model_t& m, const model_layout& L)
+// False: no gates (too large a network, or logic that is not made of AND, OR, XOR and NOT).
+bool emit_gates(std::ostream& ss, const model_t& m, const model_layout& L)
 {
 	if (!L.incremental_ok)
-		return;
+		return false;
 	const gate_network net = build_gates(m);
 	if (!net.ok)
-		return;
+		return false;
 	ss << std::endl << "// ---- lockstep kernels" << std::endl;
 	ss << "#define MBG_GATES 1" << std::endl;
 	ss << "constexpr int mbg_gate_rounds = " << net.rounds << ";" << std::endl;
@@ -479,7 +481,7 @@ void emit_gates(std::ostream& ss, const model_t& m, const model_layout& L)
 		low = std::min(low, e - 24 + __builtin_ctz((unsigned)std::ldexp(f, 24)));
 	}
 	if (values.empty() || values.size() > 3 || !std::isfinite(sum) || std::ldexp(sum, -low) > 16777216.0)
-		return;
+		return true;
 	ss << "#define MBG_RATE_CLASSES " << values.size() << std::endl;
 	ss << "__device__ __forceinline__ constexpr float mbg_class_rate(int d)" << std::endl << "{" << std::endl << "    return ";
 	for (size_t d = 0; d < values.size(); d++)
@@ -506,6 +508,14 @@ void emit_gates(std::ostream& ss, const model_t& m, const model_layout& L)
 			   << ") & " << up << "u)));" << std::endl;
 		}
 	ss << "}" << std::endl;
+	return true;
+}
+
+// Dependent records (16 bytes), dependents (8 bytes a node) and rates (8 bytes for 33 entries a state word),
+// in multiples of 16.
+size_t table_bytes(const model_layout& L)
+{
+	return (16 * L.dep_idx.size() + 8 * (size_t)L.state_size + 264 * (size_t)L.state_words + 15) / 16 * 16;
 }
 
 // forward-mode derivative of the float evaluation (expressions.cpp evaluate) w.r.t. one variable
@@ -1087,7 +1097,20 @@ std::string generate_code(const model_t& m)
 	ss << "    return h > 0.f ? h : 0.f;" << std::endl << "}" << std::endl;
 
 	emit_incremental_tables(ss, L);
-	emit_gates(ss, m, L);
+	if (!emit_gates(ss, m, L) && L.incremental_ok)
+	{
+		// the fused kernels' tables in shared memory, if at least 256 threads' rows fit beside them and the
+		// entropy sums (640 threads at most: 102 registers each)
+		const size_t smem = 227 * 1024, tables = table_bytes(L);
+		const size_t h = (size_t)L.windows() * 8 <= 48 * 1024 ? (size_t)L.windows() * 8 : 0;
+		const size_t threads = tables + h < smem ? (smem - tables - h) / ((size_t)12 * L.state_words) / 32 * 32 : 0;
+		if (threads >= 256)
+		{
+			ss << "#define MBG_TABLE_THREADS " << std::min<size_t>(threads, 640) << std::endl;
+			ss << "constexpr int mbg_table_threads = " << std::min<size_t>(threads, 640) << ";" << std::endl;
+			ss << "constexpr int mbg_table_bytes = " << tables << ";" << std::endl;
+		}
+	}
 	return ss.str();
 }
 

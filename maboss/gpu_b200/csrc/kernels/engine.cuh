@@ -267,6 +267,12 @@ __device__ __forceinline__ mb_idx_t mb_or_all(mb_idx_t v)
 #endif
 }
 
+#ifdef MBG_TABLE_THREADS
+#define MB_FUSED_BOUNDS(threads, blocks) __launch_bounds__(MBG_TABLE_THREADS, 1)
+#else
+#define MB_FUSED_BOUNDS(threads, blocks) __launch_bounds__(threads, blocks)
+#endif
+
 struct mb_incr_view
 {
 	uint32_t* st; // [w * blockDim + t]
@@ -278,8 +284,87 @@ struct mb_incr_view
 	__device__ __forceinline__ uint32_t& Q(int w) const { return ws[w * stride]; }
 };
 
+// A view with the model's tables (dependent records, dependents, rates) in the block's shared memory, where they
+// fit beside the lanes' rows (generated MBG_TABLE_THREADS: the threads of a block, one block an SM). From global
+// memory they share the L1 that the rows leave: with the rows of 512 trajectories of the 1000-node network
+// 28 KB for 55 KB of tables, half of the loads missing it; and 448 trajectories with the tables are more
+// than the 384 that leave room for them in L1. Fast mode, 1e6 trajectories: 232 -> 181 ms.
+struct mb_tab_view : mb_incr_view
+{
+	const uint4* crec;
+	const uint2* dep;
+	const uint2* q; // fast mode: integer rates, exact mode: float rates (up, down)
+};
+
+__device__ __forceinline__ uint4 mb_rec(const mb_incr_view&, int r) { return __ldg(mbg_inc_crec + r); }
+__device__ __forceinline__ uint4 mb_rec(const mb_tab_view& v, int r) { return v.crec[r]; }
+__device__ __forceinline__ uint2 mb_deps(const mb_incr_view&, int j)
+{
+	return __ldg(reinterpret_cast<const uint2*>(mbg_inc_dep) + j);
+}
+__device__ __forceinline__ uint2 mb_deps(const mb_tab_view& v, int j) { return v.dep[j]; }
+__device__ __forceinline__ uint2 mb_q(const mb_incr_view&, int j)
+{
+	return __ldg(reinterpret_cast<const uint2*>(mbg_inc_q) + j);
+}
+__device__ __forceinline__ uint2 mb_q(const mb_tab_view& v, int j) { return v.q[j]; }
+// float rate of node b of word w switching off (on = 1) or on (exact mode's table has 33 entries a word, the last
+// one zeros)
+__device__ __forceinline__ float mb_rate(const mb_incr_view&, int w, int b, unsigned on)
+{
+	return __ldg(mbg_inc_rate + 2 * (32 * w + b) + on);
+}
+__device__ __forceinline__ float mb_rate(const mb_tab_view& v, int w, int b, unsigned on)
+{
+	return reinterpret_cast<const float*>(v.q)[2 * (33 * w + b) + on];
+}
+
+// The block's shared memory: tables, then the lanes' rows (state words, unstable masks, word sums), then the
+// entropy sums (returned).
+#ifdef MBG_TABLE_THREADS
+typedef mb_tab_view mb_fused_view;
+#else
+typedef mb_incr_view mb_fused_view;
+#endif
+template <bool EXACT>
+__device__ __forceinline__ long long* mb_fused_rows(mb_fused_view& v, uint32_t* smem)
+{
+	const int B = blockDim.x;
+#ifdef MBG_TABLE_THREADS
+	uint32_t* to = smem;
+	const uint32_t* rec = reinterpret_cast<const uint32_t*>(mbg_inc_crec);
+	for (int i = threadIdx.x; i < 4 * mbg_inc_records; i += B)
+		to[i] = __ldg(rec + i);
+	to += 4 * mbg_inc_records;
+	for (int i = threadIdx.x; i < 2 * state_size; i += B)
+		to[i] = __ldg(mbg_inc_dep + i);
+	to += 2 * state_size;
+	if (EXACT)
+		for (int i = threadIdx.x; i < 66 * state_words; i += B)
+		{
+			const int w = i / 66, e = i - 66 * w;
+			const bool node = e < 64 && 64 * w + e < 2 * state_size;
+			to[i] = node ? __float_as_uint(__ldg(mbg_inc_rate + 64 * w + e)) : 0u;
+		}
+	else
+		for (int i = threadIdx.x; i < 2 * state_size; i += B)
+			to[i] = __ldg(mbg_inc_q + i);
+	__syncthreads();
+	v.crec = reinterpret_cast<const uint4*>(smem);
+	v.dep = reinterpret_cast<const uint2*>(smem + 4 * mbg_inc_records);
+	v.q = v.dep + state_size;
+	smem += mbg_table_bytes / 4;
+#endif
+	v.stride = B;
+	v.st = smem + threadIdx.x;
+	v.un = smem + (size_t)state_words * B + threadIdx.x;
+	v.ws = smem + (size_t)2 * state_words * B + threadIdx.x;
+	return reinterpret_cast<long long*>(smem + (size_t)3 * state_words * B);
+}
+
 // Logic value of the node of dependent record `hdr`/`in` in the state held by view `v`.
-__device__ __forceinline__ bool mb_incr_logic(const mb_incr_view& v, int r, const uint4& rec)
+template <class V>
+__device__ __forceinline__ bool mb_incr_logic(const V& v, int r, const uint4& rec)
 {
 	const int m = (rec.x >> 16) & 31;
 	const unsigned ins[2] = { rec.z, rec.w };
@@ -355,12 +440,13 @@ __device__ __forceinline__ float mb_incr_entropy(const V& v)
 // rate, and the words, unstable masks and word sums are assembled with warp votes/reductions.
 // Returns (through the references, valid in every lane) the group sums, total and the index of
 // the non-internal state.
-__device__ __forceinline__ void mb_incr_start(const mb_fused_params& P, const mb_incr_view& v0, int col,
+template <class V>
+__device__ __forceinline__ void mb_incr_start(const mb_fused_params& P, const V& v0, int col,
 											  unsigned long long t, unsigned long long (&gs)[MB_GROUPS],
 											  unsigned long long& total, mb_idx_t& idx)
 {
 	const int lane = threadIdx.x & 31;
-	mb_incr_view v = v0;
+	V v = v0;
 	v.st = v0.st - (threadIdx.x - col);
 	v.un = v0.un - (threadIdx.x - col);
 	v.ws = v0.ws - (threadIdx.x - col);
@@ -385,9 +471,9 @@ __device__ __forceinline__ void mb_incr_start(const mb_fused_params& P, const mb
 		if (i < state_size)
 		{
 			const int r = __ldg(mbg_inc_self + i);
-			const uint4 rec = __ldg(mbg_inc_crec + r);
+			const uint4 rec = mb_rec(v, r);
 			unstable = on != mb_incr_logic(v, r, rec);
-			const uint2 qi = __ldg(reinterpret_cast<const uint2*>(mbg_inc_q) + i);
+			const uint2 qi = mb_q(v, i);
 			q = unstable ? (on ? qi.y : qi.x) : 0u;
 			const int pos = (int)((rec.x >> 21) & 127u) - 1;
 			nibit = (pos >= 0 && on) ? ((mb_idx_t)1 << pos) : (mb_idx_t)0;
@@ -563,45 +649,18 @@ __device__ __forceinline__ bool mb_lock_ni_changed(const mb_lock& v, const uint3
 // search over the word-end sums (non-decreasing, all rates being >= 0) and a scan of one word from
 // the previous word-end sum, which reproduces the reference's running comparisons exactly.
 
-// Running fp32 sum over the unstable nodes of state word w, in node order, starting from `run`,
-// four nodes per iteration: their rate loads and bit arithmetic are independent of the chain of
-// adds (+9.8 % on the 1000-node network over two per iteration; adds of 0.f for the missing nodes
-// of a group of four leave a non-negative sum unchanged, so the sums are the same).
-__device__ __forceinline__ float mb_exact_word_sum(float run, uint32_t um, uint32_t sw, int w)
-{
-	while (um)
-	{
-		const int b0 = __ffs(um) - 1;
-		um &= um - 1u;
-		const int b1 = __ffs(um) - 1;
-		um &= um - 1u;
-		const int b2 = __ffs(um) - 1;
-		um &= um - 1u;
-		const int b3 = __ffs(um) - 1;
-		um &= um - 1u;
-		const float r0 = __ldg(mbg_inc_rate + 2 * (32 * w + b0) + ((sw >> b0) & 1u));
-		const float r1 = b1 >= 0 ? __ldg(mbg_inc_rate + 2 * (32 * w + b1) + ((sw >> b1) & 1u)) : 0.f;
-		const float r2 = b2 >= 0 ? __ldg(mbg_inc_rate + 2 * (32 * w + b2) + ((sw >> b2) & 1u)) : 0.f;
-		const float r3 = b3 >= 0 ? __ldg(mbg_inc_rate + 2 * (32 * w + b3) + ((sw >> b3) & 1u)) : 0.f;
-		run += r0;
-		run += r1;
-		run += r2;
-		run += r3;
-	}
-	return run;
-}
-
 // Unstable masks of the states held by the lanes in `lanes`, computed by the whole warp (all 32 lanes
 // call it): one node per lane, one state word at a time. Returns the calling lane's non-internal
 // index when the lane is in `lanes`, else `idx`.
-__device__ __forceinline__ mb_idx_t mb_exact_masks(const mb_incr_view& v, unsigned lanes, mb_idx_t idx)
+template <class V>
+__device__ __forceinline__ mb_idx_t mb_exact_masks(const V& v, unsigned lanes, mb_idx_t idx)
 {
 	const int lane = threadIdx.x & 31;
 	while (lanes)
 	{
 		const int src = __ffs(lanes) - 1;
 		lanes &= lanes - 1u;
-		mb_incr_view c = v;
+		V c = v;
 		c.st = v.st - (lane - src);
 		c.un = v.un - (lane - src);
 		mb_idx_t ix = 0;
@@ -614,7 +673,7 @@ __device__ __forceinline__ mb_idx_t mb_exact_masks(const mb_incr_view& v, unsign
 			if (i < state_size)
 			{
 				const int r = __ldg(mbg_inc_self + i);
-				const uint4 hdr = __ldg(mbg_inc_crec + r);
+				const uint4 hdr = mb_rec(v, r);
 				unstable = on != mb_incr_logic(c, r, hdr);
 				const int pos = (int)((hdr.x >> 21) & 127u) - 1;
 				nibit = (pos >= 0 && on) ? ((mb_idx_t)1 << pos) : (mb_idx_t)0;
@@ -631,20 +690,68 @@ __device__ __forceinline__ mb_idx_t mb_exact_masks(const mb_incr_view& v, unsign
 	return idx;
 }
 
-// compute_transition_rates: the total rate, re-summing the word-end sums from word `lo` on.
-__device__ __forceinline__ float mb_exact_total(const mb_incr_view& v, int lo)
+// Rates (up, down) of node b of word w; b = 32: zeros.
+__device__ __forceinline__ float2 mb_rates(const mb_incr_view&, int w, int b)
 {
-	float total = lo > 0 ? __uint_as_float(v.Q(lo - 1)) : 0.f;
-	for (int w = lo; w < state_words; w++)
+	return b < 32 ? make_float2(__ldg(mbg_inc_rate + 64 * w + 2 * b), __ldg(mbg_inc_rate + 64 * w + 2 * b + 1))
+				  : make_float2(0.f, 0.f);
+}
+__device__ __forceinline__ float2 mb_rates(const mb_tab_view& v, int w, int b)
+{
+	return reinterpret_cast<const float2*>(v.q)[33 * w + b];
+}
+
+// compute_transition_rates: the total rate, re-summing the word-end sums from word `lo` on: the running fp32 sum
+// over the unstable nodes in node order. One loop over chunks of at most four nodes of a word, not a loop
+// over nodes inside one over words: a lane moves on to its next word while others are still in theirs, so
+// the warp makes as many passes as its busiest lane has chunks. The word's bits are reversed once, so that the
+// next node is a count of leading zeros (32 when none is left, where the rates are zero: adding 0 to a
+// non-negative sum leaves it); the next word is loaded a pass ahead. A chunk's loads are independent of the
+// chain of adds. 1000-node network, 250,001 trajectories: 222 ms with nested loops and a find-first-set per
+// node, 194 so (two nodes a pass 206, one 250). Measured and not taken: moving the sums of unchanged words by
+// the difference of the running sums where they stay in one binade (the same sums, fewer nodes added): 255 to
+// 290 ms, each word being a chain of shared-memory loads that takes longer than adding its three nodes.
+template <class V>
+__device__ __forceinline__ float mb_exact_total(const V& v, int lo)
+{
+	float run = lo > 0 ? __uint_as_float(v.Q(lo - 1)) : 0.f;
+	int w = lo;
+	if (w >= state_words)
+		return run;
+	uint32_t um = __brev(v.U(w)), sw = __brev(v.S(w));
+	for (;;)
 	{
-		total = mb_exact_word_sum(total, v.U(w), v.S(w), w);
-		v.Q(w) = __float_as_uint(total);
+		const int wn = w + 1 < state_words ? w + 1 : w;
+		const uint32_t um_next = v.U(wn), sw_next = v.S(wn);
+		float r[4];
+#pragma unroll
+		for (int k = 0; k < 4; k++)
+		{
+			const int b = __clz(um);
+			uint32_t bit;
+			asm("shr.b32 %0, %1, %2;" : "=r"(bit) : "r"(0x80000000u), "r"(b)); // (0 for b = 32)
+			um &= ~bit;
+			const float2 both = mb_rates(v, w, b);
+			r[k] = (sw & bit) ? both.y : both.x;
+		}
+		run += r[0];
+		run += r[1];
+		run += r[2];
+		run += r[3];
+		if (um == 0)
+		{
+			v.Q(w) = __float_as_uint(run);
+			if (++w == state_words)
+				return run;
+			um = __brev(um_next);
+			sw = __brev(sw_next);
+		}
 	}
-	return total;
 }
 
 // compute_transition_entropy over the non-internal rates (generator.cpp:146-175).
-__device__ __forceinline__ float mb_exact_entropy(const mb_incr_view& v)
+template <class V>
+__device__ __forceinline__ float mb_exact_entropy(const V& v)
 {
 	float ni_total = 0.f;
 	for (int k = 0; k < mbg_noninternal_count; k++)
@@ -670,7 +777,8 @@ __device__ __forceinline__ float mb_exact_entropy(const mb_incr_view& v)
 
 // select_flip_bit: the first node whose running fp32 sum reaches r; its word is the first whose
 // word-end sum reaches r (r <= total = the last word-end sum).
-__device__ __forceinline__ int mb_exact_select(const mb_incr_view& v, float r)
+template <class V>
+__device__ __forceinline__ int mb_exact_select(const V& v, float r)
 {
 	int wl = 0, wh = state_words - 1;
 	while (wl < wh)
@@ -690,7 +798,7 @@ __device__ __forceinline__ int mb_exact_select(const mb_incr_view& v, float r)
 		const int b = __ffs(um) - 1;
 		um &= um - 1u;
 		j = 32 * wl + b;
-		sum += __ldg(mbg_inc_rate + 2 * j + ((sw >> b) & 1u));
+		sum += mb_rate(v, wl, b, (sw >> b) & 1u);
 		if (!(sum < r))
 			break;
 	}
@@ -700,11 +808,12 @@ __device__ __forceinline__ int mb_exact_select(const mb_incr_view& v, float r)
 // Flips node j, re-evaluates it and the nodes whose logic reads it, updates the non-internal index;
 // returns the lowest state word whose rates changed, and sets ni_changed when the rate of a
 // non-internal node may have changed (the transition entropy depends on nothing else).
-__device__ __forceinline__ int mb_exact_flip(const mb_incr_view& v, int j, mb_idx_t& idx, bool& ni_changed)
+template <class V>
+__device__ __forceinline__ int mb_exact_flip(const V& v, int j, mb_idx_t& idx, bool& ni_changed)
 {
 	v.S(j >> 5) ^= 1u << (j & 31);
 	int lo = j >> 5;
-	const uint2 nj = __ldg(reinterpret_cast<const uint2*>(mbg_inc_dep) + j);
+	const uint2 nj = mb_deps(v, j);
 	const int pj = (int)(nj.y >> 16) - 1;
 	if (pj >= 0)
 		idx ^= (mb_idx_t)1 << pj;
@@ -727,8 +836,8 @@ __device__ __forceinline__ int mb_exact_flip(const mb_incr_view& v, int j, mb_id
 	for (int d = d0; d < d1; d += 2)
 	{
 		const bool two = d + 1 < d1;
-		const uint4 h0 = __ldg(mbg_inc_crec + d);
-		const uint4 h1 = two ? __ldg(mbg_inc_crec + d + 1) : make_uint4(0u, 0u, 0u, 0u);
+		const uint4 h0 = mb_rec(v, d);
+		const uint4 h1 = two ? mb_rec(v, d + 1) : make_uint4(0u, 0u, 0u, 0u);
 		dependent(d, h0);
 		if (two)
 			dependent(d + 1, h1);
@@ -1036,14 +1145,14 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_exact
 #else
 // Exact mode: persistent, one thread = one trajectory at a time, with the reference's 100-slot epoch
 // boundary (every traj_len - 1 steps the same state is re-evaluated with a fresh draw).
-extern "C" __global__ void __launch_bounds__(128) mb_fused_exact(mb_fused_params P)
+extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_params P)
 {
-	extern __shared__ uint32_t mb_smem_u32[];
+	extern __shared__ __align__(16) uint32_t mb_smem_u32[];
 	const int B = blockDim.x;
 	const int lane = threadIdx.x & 31;
-	const mb_incr_view v = mb_exact_view(mb_smem_u32);
+	mb_fused_view v;
 	long long* hsink = P.st.win_h;
-	long long* smem_h = reinterpret_cast<long long*>(mb_smem_u32 + (size_t)3 * state_words * B);
+	long long* smem_h = mb_fused_rows<true>(v, mb_smem_u32);
 	if (P.st.h_in_smem)
 	{
 		for (int i = threadIdx.x; i < P.st.n_windows; i += B)
@@ -1441,18 +1550,14 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_fast(
 // at least 5 resident blocks of 128: 89 registers on the 1000-node network, no spills. Measured
 // (autotuned shapes): the 1000-node network runs equally at 4 and 5 (shared memory limits it to 3
 // or 4 blocks), the 50-node network 5.6 % faster at 5; at 6 the 1000-node network loses 11 %.
-extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_params P)
+extern "C" __global__ void MB_FUSED_BOUNDS(128, 5) mb_fused_fast(mb_fused_params P)
 {
-	extern __shared__ uint32_t mb_smem_u32[];
+	extern __shared__ __align__(16) uint32_t mb_smem_u32[];
 	const int B = blockDim.x;
 	const int lane = threadIdx.x & 31;
-	mb_incr_view v;
-	v.stride = B;
-	v.st = mb_smem_u32 + threadIdx.x;
-	v.un = mb_smem_u32 + (size_t)state_words * B + threadIdx.x;
-	v.ws = mb_smem_u32 + (size_t)2 * state_words * B + threadIdx.x;
+	mb_fused_view v;
 	long long* hsink = P.st.win_h;
-	long long* smem_h = reinterpret_cast<long long*>(mb_smem_u32 + (size_t)3 * state_words * B);
+	long long* smem_h = mb_fused_rows<false>(v, mb_smem_u32);
 	if (P.st.h_in_smem)
 	{
 		for (int i = threadIdx.x; i < P.st.n_windows; i += B)
@@ -1618,7 +1723,6 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 				const uint32_t sw = v.S(word);
 				uint32_t um = v.U(word);
 				int j = 32 * word + 31 - __clz(um | 1u);
-				const uint2* q2 = reinterpret_cast<const uint2*>(mbg_inc_q);
 				// the chosen word's unstable nodes two at a time: both rate loads are issued before
 				// the first comparison (+1.9 % on the 1000-node network over one load per step)
 				while (um)
@@ -1626,8 +1730,8 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 					const int b0 = __ffs(um) - 1;
 					const uint32_t um1 = um & (um - 1u);
 					const int b1 = um1 ? __ffs(um1) - 1 : b0;
-					const uint2 qq0 = __ldg(q2 + 32 * word + b0);
-					const uint2 qq1 = __ldg(q2 + 32 * word + b1);
+					const uint2 qq0 = mb_q(v, 32 * word + b0);
+					const uint2 qq1 = mb_q(v, 32 * word + b1);
 					const uint32_t qa = ((sw >> b0) & 1u) ? qq0.y : qq0.x;
 					j = 32 * word + b0;
 					if (r < cum + qa)
@@ -1642,7 +1746,7 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 					cum += qb;
 					um = um1 & (um1 - 1u);
 				}
-				const uint2 nj = __ldg(reinterpret_cast<const uint2*>(mbg_inc_dep) + j);
+				const uint2 nj = mb_deps(v, j);
 
 				// flip j and re-evaluate it and the nodes whose logic reads it
 				v.S(j >> 5) ^= 1u << (j & 31);
@@ -1655,7 +1759,7 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 				// independently, two at a time so that both records' loads are in flight together
 				auto dependent = [&](int d, const uint4& rec) {
 					const int k = (int)(rec.x & 0xffffu);
-					const uint2 qk = __ldg(q2 + k);
+					const uint2 qk = mb_q(v, k);
 					const int wk = k >> 5;
 					const uint32_t bk = 1u << (k & 31);
 					const bool on = (v.S(wk) & bk) != 0;
@@ -1680,8 +1784,8 @@ extern "C" __global__ void __launch_bounds__(128, 5) mb_fused_fast(mb_fused_para
 				for (int d = d0; d < d1; d += 2)
 				{
 					const bool two = d + 1 < d1;
-					const uint4 rec0 = __ldg(mbg_inc_crec + d);
-					const uint4 rec1 = two ? __ldg(mbg_inc_crec + d + 1) : make_uint4(0u, 0u, 0u, 0u);
+					const uint4 rec0 = mb_rec(v, d);
+					const uint4 rec1 = two ? mb_rec(v, d + 1) : make_uint4(0u, 0u, 0u, 0u);
 					dependent(d, rec0);
 					if (two)
 						dependent(d + 1, rec1);

@@ -426,6 +426,8 @@ std::unique_ptr<module> compile_module(context& ctx, const std::string& generate
 					 generated_code.find("#define MBG_INCREMENTAL_MANY 1") != std::string::npos;
 	m->integer_rates = generated_code.find("#define MBG_INTEGER_RATES 1") != std::string::npos;
 	m->gate_words = parse_constexpr(generated_code, "mbg_gate_words", 0);
+	m->table_threads = parse_constexpr(generated_code, "mbg_table_threads", 0);
+	m->table_bytes = (size_t)parse_constexpr(generated_code, "mbg_table_bytes", 0);
 	m->source = generated_code;
 	// the fast family is compiled now so that errors in the generated code surface here
 	m->ensure(FAMILY_FAST);
@@ -1117,6 +1119,12 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 		// per thread in shared memory: state words, unstable masks and word rate sums; or per warp its array
 		constexpr size_t max_smem = 227 * 1024;
 		block = std::min(block, 128);
+		if (m.table_threads && c.blocks_per_sm <= 0)
+		{
+			// one block an SM with all that fits; in a small run only the warps that it needs on each SM
+			const long long lanes = lanes_per_warp(n, m.ctx->sm_count), warps = (n + lanes - 1) / lanes;
+			block = (int)std::min<long long>(m.table_threads, 32 * ((warps + m.ctx->sm_count - 1) / m.ctx->sm_count));
+		}
 		while (block > 32 && m.fused_smem(block) + smem > max_smem)
 			block -= 32;
 		if (m.fused_smem(block) + smem > max_smem)
@@ -1166,9 +1174,10 @@ void simulate_epoch(module& m, bool dense, cudaStream_t s, int n, int stride, in
 	// per thread in shared memory: state words, unstable masks, word-end running sums; or per warp its array
 	constexpr size_t max_smem = 227 * 1024;
 	int block = 128;
-	while (block > 32 && m.fused_smem(block) > max_smem)
+	auto bytes = [&](int b) { return m.fused_smem(b) - m.table_bytes; }; // (its tables are in global memory)
+	while (block > 32 && bytes(block) > max_smem)
 		block -= 32;
-	const size_t smem = m.fused_smem(block);
+	const size_t smem = bytes(block);
 	if (smem > max_smem)
 		throw engine_error(MB_ERR_LIMIT, "model too large for the incremental epoch kernel's shared memory");
 	launch(m.sim_epoch, (n + block - 1) / block, block, smem, s, a);
@@ -1388,6 +1397,8 @@ std::vector<tuned_shape> autotune(module& m, const run_config& c)
 	// per state word and thread; the dense kernels any multiple of 32 up to 256
 	std::vector<std::pair<int, int>> cands;
 	const bool incr = c.mode == MB_MODE_FUSED_EXACT ? m.incremental : m.fast_incremental();
+	if (incr && m.table_threads)
+		cands.push_back({ 256, 0 }); // the kernel's own shape (mbg_table_threads, one block an SM)
 	const std::vector<int> blocks = incr ? std::vector<int>{ 128, 96, 64 } : std::vector<int>{ 256, 128 };
 	for (int block : blocks)
 	{
@@ -1408,7 +1419,7 @@ std::vector<tuned_shape> autotune(module& m, const run_config& c)
 	// a slice of the run: four times what the largest candidate keeps resident, at most the run itself
 	long long resident = 0;
 	for (auto& cd : cands)
-		resident = std::max(resident, (long long)cd.first * cd.second * m.ctx->sm_count);
+		resident = std::max(resident, (long long)(cd.second ? cd.first * cd.second : m.table_threads) * m.ctx->sm_count);
 	run_config probe = c;
 	probe.sample_count = std::max(1LL, std::min(c.sample_count, 4 * resident));
 	probe.stats_trajectories = 0;

@@ -178,10 +178,14 @@ struct module
 	bool fast_incremental() const { return incremental && integer_rates; }
 	// words of a warp's array in the lockstep kernels (generated MBG_GATES), 0: the incremental kernels
 	int gate_words = 0;
+	// threads of a block of the fused incremental kernels with their tables in shared memory and the tables'
+	// bytes (generated MBG_TABLE_THREADS), 0: tables in global memory
+	int table_threads = 0;
+	size_t table_bytes = 0;
 	// dynamic shared memory of a block of a fused incremental kernel, without the entropy sums
 	size_t fused_smem(int block) const
 	{
-		return gate_words ? (size_t)4 * gate_words * (block / 32) : (size_t)12 * state_words * block;
+		return gate_words ? (size_t)4 * gate_words * (block / 32) : table_bytes + (size_t)12 * state_words * block;
 	}
 	bool has_layout = false; // compiled from a model (full layout known)
 	model_layout layout;
