@@ -205,11 +205,7 @@ __device__ __forceinline__ void mb_fused_body(const mb_fused_params& P)
 		const unsigned long long id = P.first_traj + t;
 		if (EXACT)
 		{
-			curandState rng;
-			if (P.rands)
-				rng = static_cast<const curandState*>(P.rands)[t];
-			else
-				curand_init(P.seed, id, 0ull, &rng);
+			curandState rng = static_cast<const curandState*>(P.rands)[t];
 			mb_trajectory<true>(P, rng, hsink, trans, acc);
 		}
 		else
@@ -1026,18 +1022,10 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_exact
 			if (t < P.n_traj)
 			{
 				starting = true;
-				if (P.rands)
-					rng = static_cast<const curandState*>(P.rands)[t];
-				else
-					curand_init(P.seed, P.first_traj + t, 0ull, &rng);
-				if (P.init_states) // drawn by the init launch
-				{
+				rng = static_cast<const curandState*>(P.rands)[t];
 #pragma unroll
-					for (int w = 0; w < MB_LW; w++)
-						v.s[w] = __ldg(P.init_states + (size_t)w * P.n_traj + t);
-				}
-				else
-					mb_init_state(v.s, rng, P.istate);
+				for (int w = 0; w < MB_LW; w++)
+					v.s[w] = __ldg(P.init_states + (size_t)w * P.n_traj + t);
 #pragma unroll
 				for (int w = 0; w < MB_LW; w++)
 					v.u[w] = 0u, q[w] = 0.f;
@@ -1182,25 +1170,10 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_param
 			if (t < P.n_traj)
 			{
 				starting = true;
-				// curand_init's skip-ahead is long and a lane starting a trajectory would run it while
-				// the rest of its warp waits: the states come from a parallel init launch when given
-				if (P.rands)
-					rng = static_cast<const curandState*>(P.rands)[t];
-				else
-					curand_init(P.seed, P.first_traj + t, 0ull, &rng);
-				if (P.init_states) // drawn by the init launch
-					for (int w = 0; w < state_words; w++)
-						v.S(w) = __ldg(P.init_states + (size_t)w * P.n_traj + t);
-				else // one uniform per node in node order (simulation.cu:51-53)
+				// random state and initial state as the init launch left them
+				rng = static_cast<const curandState*>(P.rands)[t];
 				for (int w = 0; w < state_words; w++)
-				{
-					uint32_t sw = 0;
-					const int nb = (w == state_words - 1) ? state_size - 32 * w : 32;
-					for (int b = 0; b < nb; b++)
-						if (curand_uniform(&rng) <= __ldg(P.istate + 32 * w + b))
-							sw |= 1u << b;
-					v.S(w) = sw;
-				}
+					v.S(w) = __ldg(P.init_states + (size_t)w * P.n_traj + t);
 			}
 			else
 				working = false;

@@ -61,6 +61,6 @@ struct mb_fused_params
 	unsigned long long* transitions; // executed simulate iterations
 	unsigned* errors;				 // trajectories stopped because the total rate was not finite
 	void* rands;					 // exact mode: curandState of trajectory t at [t], initialised by a
-									 // separate mb_initialize_random launch, or null (curand_init inline)
-	const unsigned* init_states;	 // exact mode: initial states [word * n_traj + t] that the launch drew, or null
+									 // separate mb_initialize_random launch
+	const unsigned* init_states;	 // incremental exact mode: initial states [word * n_traj + t] that it drew
 };

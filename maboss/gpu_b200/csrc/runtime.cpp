@@ -1079,8 +1079,6 @@ namespace {
 unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long n, cudaStream_t s, void* rng,
 					  unsigned* init_states)
 {
-	if (n > 0xffffffffLL)
-		throw engine_error(MB_ERR_LIMIT, "sample_count above 2^32 - 1");
 	if (n == 0)
 		return 0;
 	mb_fused_params P{};
@@ -1334,11 +1332,14 @@ runner::runner(module& m, const run_config& c) : mod(&m), cfg(c)
 	st.init(m, c.time_tick, c.max_time, c.discrete_time, c.noninternal_nodes, c.sample_count, c.fixed_capacity_log2, s,
 			7u, c.stats_trajectories, c.bin_capacity_log2);
 	st.set_istate(c.istate, s);
-	if (c.mode == MB_MODE_FUSED_EXACT && c.sample_count > 0 && c.sample_count <= max_rng_states)
+	if (c.mode == MB_MODE_FUSED_EXACT && c.sample_count > 0)
 	{
-		rng.alloc((size_t)c.sample_count * sizeof(curandState));
-		if (m.incremental && 4 * m.state_words * c.sample_count <= max_init_bytes)
-			init_states.alloc((size_t)4 * m.state_words * c.sample_count);
+		rng_chunk = std::min(c.sample_count, max_rng_states);
+		if (m.incremental)
+			rng_chunk = std::max(1LL, std::min(rng_chunk, max_init_bytes / (4 * m.state_words)));
+		rng.alloc((size_t)rng_chunk * sizeof(curandState));
+		if (m.incremental)
+			init_states.alloc((size_t)4 * m.state_words * rng_chunk);
 	}
 	MB_CUDA(cudaEventCreate(&ev0));
 	MB_CUDA(cudaEventCreate(&ev1));
@@ -1371,7 +1372,17 @@ void runner::launch(cudaStream_t s)
 	}
 	else
 	{
-		launches = launch_fused(*mod, cfg, st, cfg.sample_count, s, rng.p, init_states.as<unsigned>());
+		if (cfg.sample_count > 0xffffffffLL)
+			throw engine_error(MB_ERR_LIMIT, "sample_count above 2^32 - 1");
+		run_config c = cfg;
+		const long long chunk = rng_chunk > 0 ? rng_chunk : std::max(1LL, cfg.sample_count);
+		for (long long done = 0; done < cfg.sample_count; done += chunk)
+		{
+			if (done)
+				MB_CUDA(cudaMemsetAsync(st.next_traj(), 0, sizeof(unsigned long long), s));
+			c.first_traj = cfg.first_traj + (unsigned long long)done;
+			launches += launch_fused(*mod, c, st, std::min(chunk, cfg.sample_count - done), s, rng.p, init_states.as<unsigned>());
+		}
 		epochs = 1;
 	}
 	MB_CUDA(cudaEventRecord(ev1, s));

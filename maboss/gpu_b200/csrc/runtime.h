@@ -403,11 +403,12 @@ struct runner
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 	int epochs = 0;
 	unsigned launches = 0; // engine kernels enqueued by the last launch()
-	dbuf rng;			   // exact mode: XORWOW states of every trajectory (empty above max_rng_states)
+	// exact mode: XORWOW states and (incremental kernels) initial states of the trajectories of a launch. A run of
+	// more is several launches: the kernels start every trajectory from these, as curand_init in them, for
+	// the runs without, took 96 registers and a stack frame
+	dbuf rng, init_states;
+	long long rng_chunk = 0; // trajectories of a launch
 	static constexpr long long max_rng_states = 1LL << 24;
-	// incremental exact mode: initial states of every trajectory (empty where they take more than 1 GB:
-	// the kernel then draws them itself)
-	dbuf init_states;
 	static constexpr long long max_init_bytes = 1LL << 30;
 	// epoch modes: kept for the next launch where they take at most 4 GB (allocating and freeing the 0.2 GB of
 	// 1e5 trajectories of the 87-node example model took 9 to 20 ms a run), else given back after each run

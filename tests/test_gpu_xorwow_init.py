@@ -28,3 +28,16 @@ def test_initial_states_of_several_words(gpu):
         res = gpu.compile(mb.Model(bnd, cfg)).run(mode=mode, sample_count=5_003, seed=4)
         ref = OracleModel(bnd, cfg).run(n=5_003, mode=0, seed=4)
         assert res.transitions == ref["transitions"] and np.array_equal(res.final_counts, ref["final"])
+
+
+def test_runs_of_several_launches(gpu):
+    """More trajectories than the random states that are kept (2^24): several launches, the same sums as two runs."""
+    mod = gpu.compile(mb.Model(*synth.c1()))
+    n, first = (1 << 24) + 1000, 1 << 24
+    whole = mod.run(mode="exact", sample_count=n, seed=2)
+    parts = [mod.run(mode="exact", sample_count=k, seed=2, first_traj=f, stats_trajectories=n)
+             for k, f in ((first, 0), (1000, first))]
+    merged = mb.merge_results(parts)
+    assert whole.transitions == merged.transitions
+    assert np.array_equal(whole.final_counts, merged.final_counts)
+    assert np.array_equal(whole.raw()["occ"], merged.raw()["occ"])
