@@ -400,6 +400,8 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 		N.mod->ensure(FAMILY_BATCH);
 		ps->fn = grad ? N.mod->batched_grad_static : N.mod->batched_fast_static;
 		ps->smem_per_warp = (size_t)4 * N.mod->gate_words;
+		if (N.mod->gate_words && vars_.size() == 1 && vars_[0]->st.n_windows <= 1024)
+			B.h_windows = vars_[0]->st.n_windows;
 	}
 	ps->smem_per_thread = ((ps->smem_per_warp ? 0 : 3 * (size_t)max_W) + (grad ? 2 * (size_t)P : 0)) * 4;
 	MB_CUDA(cudaStreamSynchronize(s));
@@ -411,7 +413,7 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 int batch_engine::fit(prepared& ps, int block, size_t& smem) const
 {
 	constexpr size_t max_smem = 227 * 1024;
-	smem = (size_t)block * ps.smem_per_thread + (size_t)(block / 32) * ps.smem_per_warp;
+	smem = (size_t)block * ps.smem_per_thread + (size_t)(block / 32) * ps.smem_per_warp + (size_t)ps.B->h_windows * sizeof(long long);
 	if (smem > max_smem)
 		return 0;
 	if (smem > 48 * 1024)

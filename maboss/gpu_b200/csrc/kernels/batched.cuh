@@ -60,6 +60,7 @@ struct mb_batch_params
 	int max_W;			  // shared memory rows per lane
 	int P;				  // gradient parameters (rows of gradient scratch), 0 = none
 	unsigned long long total;
+	int h_windows;		  // one variant, lockstep kernels: windows of its entropy sums in shared memory (0: global)
 	int lanes;			  // lanes of each warp that take trajectories (fewer than 32 in small runs)
 	unsigned long long seed;
 	unsigned long long* next;
@@ -292,15 +293,15 @@ __device__ __forceinline__ void mbb_grad_slice(const mb_variant& var, const mbb_
 }
 
 template <bool GRAD>
-__device__ __forceinline__ void mbb_record(const mb_variant& var, const mbb_lane& v, int P, mb_win_acc& acc,
-										   unsigned idx, float t0, float t1, float h, bool fixed, bool discrete,
+__device__ __forceinline__ void mbb_record(const mb_variant& var, long long* hsink, const mbb_lane& v, int P,
+										   mb_win_acc& acc, unsigned idx, float t0, float t1, float h, bool fixed, bool discrete,
 										   float tick, double& C1, double& C2, mbb_cot_cache& cc)
 {
 	if (t1 == 0.f)
 		return;
 	if (discrete)
 	{
-		mb_record_disc(var.st, var.st.win_h, idx, t0, h);
+		mb_record_disc(var.st, hsink, idx, t0, h);
 		if (GRAD)
 		{
 			const int w = (int)lroundf(t0 / tick);
@@ -309,10 +310,18 @@ __device__ __forceinline__ void mbb_record(const mb_variant& var, const mbb_lane
 		}
 		return;
 	}
+	if (GRAD && !fixed)
+	{
+		// the gradient's slices with the window sums' (one loop)
+		mb_record_slices(acc, var.st, hsink, idx, t0, t1, h, [&](int w, float sb, float se) {
+			mbb_grad_slice(var, v, P, w, idx, sb, se, false, C1, C2, cc);
+		});
+		return;
+	}
 	if (fixed)
-		mb_record_fixed(acc, var.st, var.st.win_h, idx, t0, t1);
+		mb_record_fixed(acc, var.st, hsink, idx, t0, t1);
 	else
-		mb_record_cont(acc, var.st, var.st.win_h, idx, t0, t1, h);
+		mb_record_cont(acc, var.st, hsink, idx, t0, t1, h);
 	if (GRAD)
 	{
 		// the same window slices as mb_record_cont
@@ -511,7 +520,7 @@ __device__ void mbb_body(const mb_batch_params& B)
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				mbb_record<GRAD>(var, v, P, acc, idx, time, max_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
+				mbb_record<GRAD>(var, var.st.win_h, v, P, acc, idx, time, max_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
 				atomicAdd(var.st.final_cnt + idx, 1u);
 				unsigned st[64];
 				const int W = net.W() < 64 ? net.W() : 64;
@@ -538,7 +547,7 @@ __device__ void mbb_body(const mb_batch_params& B)
 			}
 			tn = fminf(tn, max_time);
 			trans += (tn != 0.f) ? 1ull : 0ull;
-			mbb_record<GRAD>(var, v, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
+			mbb_record<GRAD>(var, var.st.win_h, v, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
 			time = tn;
 			if (time >= max_time)
 			{
@@ -708,7 +717,7 @@ struct mbb_net_static
 // The batched algorithm on lockstep logic (networks of at most 256 nodes, kernels/engine.cuh): the same random
 // numbers, rates, choices and order of the score's updates as mbb_body. Shared memory: the warps' arrays,
 // then the gradient's A_p and D_p of every thread. Forward and gradient of the 50-node network with 40
-// parameters, 1e6 trajectories, end to end 31.6 -> 25.0 ms.
+// parameters, 1e6 trajectories, end to end 31.6 -> 25.0 ms, 21.6 with the steps below.
 template <bool GRAD>
 __device__ void mbb_lock_body(const mb_batch_params& B)
 {
@@ -725,6 +734,15 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 	g.gD = gbase + (size_t)P * bs + threadIdx.x;
 	g.gstride = B.gstride;
 	g.gR = GRAD ? B.gmem + blockIdx.x * bs + threadIdx.x : nullptr;
+	// one variant: its entropy sums per block (its few windows are every lane's, so their global adds meet)
+	long long* smem_h = nullptr;
+	if (B.h_windows)
+	{
+		smem_h = reinterpret_cast<long long*>(gbase + (size_t)2 * P * bs);
+		for (int i = threadIdx.x; i < B.h_windows; i += bs)
+			smem_h[i] = 0;
+		__syncthreads();
+	}
 	double C1 = 0.0, C2 = 0.0; // continuous-time gradient running sums of the lane's trajectory
 	for (int p = 0; p < P; p++)
 	{
@@ -750,13 +768,24 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 	unsigned long long trans = 0;
 	curandStatePhilox4_32_10_t rng;
 
-	while (__any_sync(0xffffffffu, working || running))
+	bool ended = false; // gradient: the lane's last trajectory is not added to R_p yet
+	for (;;)
 	{
+		const unsigned idle = __ballot_sync(0xffffffffu, working && !running), busy = __ballot_sync(0xffffffffu, running);
+		if (!(idle | busy))
+			break;
 		unsigned long long t = 0;
 		int tv = 0;
 		bool starting = false;
-		if (working && !running)
+		// a warp waits for some lanes to end their trajectories and start new ones together (the sums over the
+		// parameters at a trajectory's end and the start cost the warp the same for one lane as for four: 50
+		// nodes, 1e6 trajectories, gradient with 1 / 2 / 4 / 8 lanes 15.4 / 14.2 / 13.6 / 13.7 ms, forward 6.8 /
+		// 6.5 / 6.5 / 6.7)
+		if (working && !running && (__popc(idle) >= (GRAD ? 4 : 2) || !busy))
 		{
+			if (GRAD && ended)
+				mbb_grad_end(g, P, discrete, C1, C2);
+			ended = false;
 			t = atomicAdd(B.next, 1ull);
 			if (t < B.total)
 			{
@@ -817,7 +846,7 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 				{
 					if (acc_var >= 0)
 					{
-						mb_acc_flush(acc, B.vars[acc_var].st, B.vars[acc_var].st.win_h);
+						mb_acc_flush(acc, B.vars[acc_var].st, smem_h ? smem_h : B.vars[acc_var].st.win_h);
 						if (GRAD)
 							mbb_grad_emit(B.vars[acc_var], g, P);
 					}
@@ -875,15 +904,14 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				mbb_record<GRAD>(var, g, P, acc, idx, time, end_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
+				mbb_record<GRAD>(var, smem_h ? smem_h : var.st.win_h, g, P, acc, idx, time, end_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
 				atomicAdd(var.st.final_cnt + idx, 1u);
 				uint32_t st[MB_LW]; // (a copy: v.s stays in registers)
 #pragma unroll
 				for (int w = 0; w < MB_LW; w++)
 					st[w] = v.s[w];
 				mb_fixed_insert_rt(var.st, st, MB_LW);
-				if (GRAD)
-					mbb_grad_end(g, P, discrete, C1, C2);
+				ended = true;
 				atomicAdd(var.transitions, trans + 1);
 				trans = 0;
 			}
@@ -904,14 +932,13 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 				}
 				tn = fminf(tn, end_time);
 				trans += (tn != 0.f) ? 1ull : 0ull;
-				mbb_record<GRAD>(var, g, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
+				mbb_record<GRAD>(var, smem_h ? smem_h : var.st.win_h, g, P, acc, idx, time, tn, h, false, discrete, var.st.win_tick, C1, C2, cc);
 				time = tn;
 				if (time >= end_time)
 				{
 					running = false;
 					atomicAdd(var.st.final_cnt + idx, 1u);
-					if (GRAD)
-						mbb_grad_end(g, P, discrete, C1, C2);
+					ended = true;
 					atomicAdd(var.transitions, trans);
 					trans = 0;
 				}
@@ -978,14 +1005,28 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 	}
 	if (acc_var >= 0)
 	{
-		mb_acc_flush(acc, B.vars[acc_var].st, B.vars[acc_var].st.win_h);
+		mb_acc_flush(acc, B.vars[acc_var].st, smem_h ? smem_h : B.vars[acc_var].st.win_h);
 		if (GRAD)
 			mbb_grad_emit(B.vars[acc_var], g, P);
+	}
+	if (smem_h)
+	{
+		__syncthreads();
+		for (int i = threadIdx.x; i < B.h_windows; i += bs)
+			if (smem_h[i] != 0)
+				atomicAdd(reinterpret_cast<unsigned long long*>(B.vars[0].st.win_h + i), (unsigned long long)smem_h[i]);
 	}
 }
 #endif // MBG_GATES
 
-extern "C" __global__ void __launch_bounds__(128, 5) mb_batched_fast_static(mb_batch_params B)
+// the lockstep forward kernel of two state words in 73 registers: 50 nodes, 1e6 trajectories 6.5 -> 5.9 ms (three
+// words and more keep the room for theirs)
+#ifdef MBG_GATES
+constexpr int MBB_FAST_BLOCKS = state_words <= 2 ? 7 : 5;
+#else
+constexpr int MBB_FAST_BLOCKS = 5;
+#endif
+extern "C" __global__ void __launch_bounds__(128, MBB_FAST_BLOCKS) mb_batched_fast_static(mb_batch_params B)
 {
 #ifdef MBG_GATES
 	mbb_lock_body<false>(B);

@@ -117,8 +117,10 @@ __device__ __forceinline__ void mb_acc_flush(mb_win_acc& a, const mb_stats_param
 
 // Continuous time: the state `idx` occupies (t0, t1]; split it over windows exactly like
 // window_average_small.cu:66-92 and add each slice (and h * slice) to its window.
-__device__ __forceinline__ void mb_record_cont(mb_win_acc& a, const mb_stats_params& p, long long* hsink,
-											   mb_idx_t idx, float t0, float t1, float h)
+// f(w, begin, end) is called for each slice.
+template <class F>
+__device__ __forceinline__ void mb_record_slices(mb_win_acc& a, const mb_stats_params& p, long long* hsink,
+												 mb_idx_t idx, float t0, float t1, float h, F f)
 {
 	float sb = t0;
 	int w = (int)floorf(sb / p.win_tick);
@@ -150,10 +152,17 @@ __device__ __forceinline__ void mb_record_cont(mb_win_acc& a, const mb_stats_par
 				a.hw = w;
 				a.hq = hq;
 			}
+			f(w, sb, se);
 		}
 		w++;
 		sb = se;
 	}
+}
+
+__device__ __forceinline__ void mb_record_cont(mb_win_acc& a, const mb_stats_params& p, long long* hsink,
+											   mb_idx_t idx, float t0, float t1, float h)
+{
+	mb_record_slices(a, p, hsink, idx, t0, t1, h, [](int, float, float) {});
 }
 
 // Continuous time, a fixed point reached at t0: the state stays until max_time, with no transition
