@@ -208,6 +208,248 @@ struct builder
 	}
 };
 
+// ---- factored forms from truth tables
+//
+// Logics of example models are written as sums of many products (153 literals for 10 inputs) of a function
+// that a dozen literals express. The table of the function (32 patterns a word; input t of `in` at bit t) is
+// split recursively: by a literal that is a factor or a term of it, else by a literal x as f = x g | h or
+// f = (x | g) & h, where g and h are only bounded from below and above, so that they lose inputs.
+
+typedef std::vector<unsigned> table;
+
+struct factoring
+{
+	std::vector<int> in; // nodes
+	static unsigned low(int t)
+	{
+		static const unsigned masks[5] = { 0xaaaaaaaau, 0xccccccccu, 0xf0f0f0f0u, 0xff00ff00u, 0xffff0000u };
+		return masks[t];
+	}
+	// f with input t fixed to v
+	static table cofactor(const table& f, int t, bool v)
+	{
+		table r(f.size());
+		for (size_t w = 0; w < f.size(); w++)
+		{
+			if (t >= 5)
+			{
+				const size_t bit = (size_t)1 << (t - 5);
+				r[w] = f[v ? w | bit : w & ~bit];
+				continue;
+			}
+			const unsigned x = v ? f[w] & low(t) : f[w] & ~low(t);
+			r[w] = v ? x | x >> (1 << t) : x | x << (1 << t);
+		}
+		return r;
+	}
+	template <class F>
+	static table map(const table& a, const table& b, F f)
+	{
+		table r(a.size());
+		for (size_t w = 0; w < a.size(); w++)
+			r[w] = f(a[w], b[w]);
+		return r;
+	}
+	static table both(const table& a, const table& b) { return map(a, b, [](unsigned x, unsigned y) { return x & y; }); }
+	static table either(const table& a, const table& b) { return map(a, b, [](unsigned x, unsigned y) { return x | y; }); }
+	static table except(const table& a, const table& b) { return map(a, b, [](unsigned x, unsigned y) { return x & ~y; }); }
+	static bool all(const table& a, unsigned v)
+	{
+		return std::all_of(a.begin(), a.end(), [&](unsigned x) { return x == v; });
+	}
+	static bool within(const table& a, const table& b) { return all(except(a, b), 0u); }
+	table of(const bexpr& e) const
+	{
+		const size_t words = (size_t)1 << (in.size() > 5 ? in.size() - 5 : 0);
+		table r(words, e.kind == bexpr::AND ? ~0u : 0u);
+		switch (e.kind)
+		{
+			case bexpr::CONST: return table(words, e.neg ? ~0u : 0u);
+			case bexpr::LIT:
+			{
+				const int t = (int)(std::find(in.begin(), in.end(), e.node) - in.begin());
+				for (size_t w = 0; w < words; w++)
+					r[w] = (t < 5 ? low(t) : (w >> (t - 5)) & 1 ? ~0u : 0u) ^ (e.neg ? ~0u : 0u);
+				return r;
+			}
+			default:
+				for (const bexpr& c : e.ch)
+				{
+					const table x = of(c);
+					for (size_t w = 0; w < words; w++)
+						r[w] = e.kind == bexpr::AND ? r[w] & x[w] : e.kind == bexpr::OR ? r[w] | x[w] : r[w] ^ x[w];
+				}
+				return r;
+		}
+	}
+	bexpr literal(int t, bool neg) const
+	{
+		bexpr e;
+		e.kind = bexpr::LIT;
+		e.node = in[t];
+		e.neg = neg;
+		return e;
+	}
+	static bexpr join(bexpr::kind_t kind, bexpr a, bexpr b)
+	{
+		bexpr r;
+		r.kind = kind;
+		for (bexpr* x : { &a, &b })
+		{
+			if (x->kind == bexpr::CONST)
+			{
+				if (x->neg == (kind == bexpr::OR))
+					return *x;
+				continue;
+			}
+			if (x->kind == kind)
+				r.ch.insert(r.ch.end(), x->ch.begin(), x->ch.end());
+			else
+				r.ch.push_back(*x);
+		}
+		if (r.ch.empty())
+		{
+			bexpr c;
+			c.neg = kind == bexpr::AND;
+			return c;
+		}
+		if (r.ch.size() == 1)
+			return bexpr(r.ch[0]);
+		return r;
+	}
+	// drops the inputs that a function between the bounds can do without
+	static void reduce(table& lo, table& hi, std::vector<int>& vars)
+	{
+		for (size_t i = 0; i < vars.size();)
+		{
+			const table l = either(cofactor(lo, vars[i], false), cofactor(lo, vars[i], true));
+			const table h = both(cofactor(hi, vars[i], false), cofactor(hi, vars[i], true));
+			if (!within(l, h))
+			{
+				i++;
+				continue;
+			}
+			lo = l;
+			hi = h;
+			vars.erase(vars.begin() + (std::ptrdiff_t)i);
+		}
+	}
+	static size_t support(table lo, table hi, std::vector<int> vars)
+	{
+		reduce(lo, hi, vars);
+		return vars.size();
+	}
+	// an expression of a function between lo and hi
+	bexpr make(table lo, table hi, std::vector<int> vars) const
+	{
+		bexpr e;
+		if (all(lo, 0u))
+			return e; // 0
+		if (all(hi, ~0u))
+		{
+			e.neg = true;
+			return e;
+		}
+		reduce(lo, hi, vars);
+		size_t best = ~(size_t)0;
+		int at = -1, form = 0;
+		for (int t : vars)
+		{
+			const table l[2] = { cofactor(lo, t, false), cofactor(lo, t, true) };
+			const table h[2] = { cofactor(hi, t, false), cofactor(hi, t, true) };
+			for (int v = 0; v < 2; v++) // the literal is true where the input is v
+			{
+				if (all(l[1 - v], 0u))
+					return join(bexpr::AND, literal(t, v == 0), make(l[v], h[v], vars));
+				if (all(h[v], ~0u))
+					return join(bexpr::OR, literal(t, v == 0), make(l[1 - v], h[1 - v], vars));
+			}
+			for (int v = 0; v < 2; v++)
+			{
+				const table hh = both(h[0], h[1]), ll = either(l[0], l[1]);
+				if (within(l[1 - v], hh))
+				{
+					const size_t c = support(l[1 - v], hh, vars) + support(except(l[v], hh), h[v], vars);
+					if (c < best)
+						best = c, at = t, form = v;
+				}
+				if (within(ll, h[v]))
+				{
+					const size_t c = support(ll, h[v], vars) + support(l[1 - v], either(h[1 - v], map(ll, ll, [](unsigned x, unsigned) { return ~x; })), vars);
+					if (c < best)
+						best = c, at = t, form = 2 + v;
+				}
+			}
+		}
+		if (at < 0) // x g | !x h
+		{
+			const int t = vars[0];
+			const bexpr g = make(cofactor(lo, t, true), cofactor(hi, t, true), vars);
+			const bexpr h = make(cofactor(lo, t, false), cofactor(hi, t, false), vars);
+			return join(bexpr::OR, join(bexpr::AND, literal(t, false), g), join(bexpr::AND, literal(t, true), h));
+		}
+		const int v = form & 1;
+		const table l[2] = { cofactor(lo, at, false), cofactor(lo, at, true) };
+		const table h[2] = { cofactor(hi, at, false), cofactor(hi, at, true) };
+		if (form < 2) // x g | rest
+		{
+			const bexpr rest = make(l[1 - v], both(h[0], h[1]), vars);
+			const bexpr g = make(except(l[v], of(rest)), h[v], vars);
+			return join(bexpr::OR, join(bexpr::AND, literal(at, v == 0), g), rest);
+		}
+		// (x | g) & rest
+		const bexpr rest = make(either(l[0], l[1]), h[v], vars);
+		const table not_rest = map(of(rest), l[0], [](unsigned x, unsigned) { return ~x; });
+		const bexpr g = make(l[1 - v], either(h[1 - v], not_rest), vars);
+		return join(bexpr::AND, join(bexpr::OR, literal(at, v == 0), g), rest);
+	}
+};
+
+void inputs_of(const bexpr& e, std::vector<int>& in)
+{
+	if (e.kind == bexpr::LIT && std::find(in.begin(), in.end(), e.node) == in.end())
+		in.push_back(e.node);
+	for (const bexpr& c : e.ch)
+		inputs_of(c, in);
+}
+
+size_t literals_of(const bexpr& e)
+{
+	size_t n = e.kind == bexpr::LIT ? 1 : 0;
+	for (const bexpr& c : e.ch)
+		n += literals_of(c);
+	return n;
+}
+
+// Intermediate gates of an expression and their levels.
+std::pair<size_t, int> cost_of(const bexpr& e)
+{
+	builder b{ 1 << 20, (1 << 20) + 1, {} };
+	b.make(e);
+	int levels = 0;
+	for (const builder::item& t : b.temps)
+		levels = std::max(levels, t.level + 1);
+	return { b.temps.size(), levels };
+}
+
+// The logic as written, or its factored form where that takes fewer gates.
+bexpr shorter(bexpr e)
+{
+	factoring f;
+	inputs_of(e, f.in);
+	if (f.in.size() < 2 || f.in.size() > 10 || literals_of(e) <= 4)
+		return e;
+	const std::pair<size_t, int> cost = cost_of(e);
+	if (cost.first <= 1)
+		return e;
+	const table t = f.of(e);
+	std::vector<int> vars(f.in.size());
+	for (size_t i = 0; i < vars.size(); i++)
+		vars[i] = (int)i;
+	bexpr g = f.make(t, t, vars);
+	return cost_of(g) < cost ? g : e;
+}
+
 } // namespace
 
 gate_network build_gates(const model_t& m)
@@ -223,7 +465,7 @@ gate_network build_gates(const model_t& m)
 	try
 	{
 		for (int i = 0; i < N; i++)
-			finals[i] = b.make(parse(m, m.nodes[i].get_attr("logic"), m.nodes[i].name));
+			finals[i] = b.make(shorter(parse(m, m.nodes[i].get_attr("logic"), m.nodes[i].name)));
 	}
 	catch (const unsupported&)
 	{

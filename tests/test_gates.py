@@ -8,6 +8,7 @@ import pytest
 
 import maboss.gpu_b200 as mb
 from oracle.oracle import OracleModel
+from conftest import model_text
 from test_codegen_host import PRELUDE
 
 WRAPPER = r"""
@@ -67,16 +68,38 @@ def model(n, values=None, seed=0, discrete=0, depth=3):
     return bnd, cfg + f"max_time = 4; time_tick = 0.3; discrete_time = {discrete}; sample_count = 1000;\n"
 
 
+@pytest.mark.parametrize("name", ["cellcycle", "sizek", "metastasis", "Montagud2022_Prostate_Cancer"])
+def test_gates_encode_the_logic_of_example_models(tmp_path, name):
+    """(logics of up to 236 literals, whose gates come from a factored form)"""
+    m = mb.Model(*model_text(name))
+    L = _gate_library(tmp_path, m.generate_code())
+    _check_gates(L, m.num_nodes, False)
+
+
 @pytest.mark.parametrize("n,values", [(1, [1.0]), (31, None), (32, [1.0, 10.0]), (33, [0.5, 0.0]), (64, None),
                                       (97, [1.0, 2.0, 4.0]), (200, None)])
 def test_gates_encode_the_logic(tmp_path, n, values):
-    code = mb.Model(*model(n, values)).generate_code()
+    L = _gate_library(tmp_path, mb.Model(*model(n, values)).generate_code())
+    assert L.host_classes() == (0 if values is None else len([v for v in values if v > 0]) if n > 1 else 1)
+    _check_gates(L, n, values is None)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_gates_of_long_logics(tmp_path, seed):
+    """Random trees of up to 32 literals of 12 nodes (factored where that is shorter), XOR and constants among them."""
+    L = _gate_library(tmp_path, mb.Model(*model(12, seed=seed, depth=5)).generate_code())
+    _check_gates(L, 12, True)
+
+
+def _gate_library(tmp_path, code):
     assert "#define MBG_GATES 1" in code
     (tmp_path / "m.cpp").write_text(PRELUDE + code + WRAPPER)
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", str(tmp_path / "m.so"),
                     str(tmp_path / "m.cpp")], check=True, timeout=300)
-    L = C.CDLL(str(tmp_path / "m.so"))
-    assert L.host_classes() == (0 if values is None else len([v for v in values if v > 0]) if n > 1 else 1)
+    return C.CDLL(str(tmp_path / "m.so"))
+
+
+def _check_gates(L, n, positive):
     rng = np.random.default_rng(1)
     for _ in range(8):
         bits = rng.random((n, 32)) < 0.5
@@ -91,7 +114,7 @@ def test_gates_encode_the_logic(tmp_path, n, values):
             L.host_rates(r.ctypes.data_as(C.c_void_p), words.ctypes.data_as(C.c_void_p))
             unstable = ((out >> np.uint32(t)) & 1).astype(bool) != bits[:, t]
             assert not (r[~unstable] != 0).any()
-            if values is None:  # (a listed rate may be 0)
+            if positive:  # (a listed rate may be 0)
                 assert (r[unstable] != 0).all()
 
 
