@@ -805,30 +805,10 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 			else
 				working = false;
 		}
-		unsigned pending = __ballot_sync(0xffffffffu, starting);
-		if (pending)
+		if (__any_sync(0xffffffffu, starting))
 		{
-			uint32_t* words = ns + 64 * MB_LW + 2; // (the gates' words)
-			while (pending)
-			{
-				const int src = __ffs(pending) - 1;
-				pending &= pending - 1u;
-				const unsigned long long ts = __shfl_sync(0xffffffffu, t, src);
-				const mb_variant& var = B.vars[__shfl_sync(0xffffffffu, tv, src)];
-				mb_philox_initial_state(B.seed, var.first_traj + (ts - var.begin), state_size, var.istate,
-										[&](int w, uint32_t word) {
-											if (lane == 0)
-												words[w] = word;
-										});
-				__syncwarp();
-				if (lane == src)
-				{
-#pragma unroll
-					for (int w = 0; w < MB_LW; w++)
-						v.s[w] = words[w];
-				}
-				__syncwarp();
-			}
+			const mb_variant& first = B.vars[tv];
+			mb_lock_start(ns, v, B.seed, first.first_traj + (t - first.begin), first.istate, starting);
 			if (starting)
 			{
 				vi = tv;

@@ -504,6 +504,14 @@ __device__ __forceinline__ void mb_incr_start(const mb_fused_params& P, const V&
 // 411 -> 221 us; 87-node one, fast, 1e5 9.3 -> 4.1 ms; 50 nodes fast 1e6 9.4 -> 5.9 ms (e); 10 nodes fast
 // 1e5 285 -> 161 us; 100 nodes (c2), 20 outputs, 2e5 15.1 -> 13.6 ms (e).
 constexpr int MB_LW = state_words;
+// Networks whose initial state a lane draws itself when some lanes start together (mb_lock_start; in larger ones
+// the code alone cost the 50-node network a block an SM).
+constexpr bool MB_LOCK_SMALL = state_size <= 36;
+// Fast mode: a warp waits for this many lanes to start together while others run. Many where trajectories are
+// short and starting together is cheap, few where the passes that idle lanes wait through are long (gates).
+// 2 / 4 / 8 lanes, ms: 10 nodes 1e6 0.85 / 0.79 / 0.75, 50 nodes 1e6 5.54 / 5.49 / 5.63, 100 nodes 2e5 3.14 /
+// 3.11 / 3.15, the 87-node example model (8 rounds of gates) 2e5 4.64 / 4.69 / 4.70.
+constexpr int MB_LOCK_STARTS = MB_LOCK_SMALL ? 8 : mbg_gate_rounds <= 2 ? 4 : 2;
 #ifndef MB_LOCK_BLOCKS
 #define MB_LOCK_BLOCKS 5
 #endif
@@ -606,6 +614,67 @@ __device__ __forceinline__ void mb_lock_flip(uint32_t* ns, mb_lock& v, int j)
 		v.s[w] ^= w == (j >> 5) ? bit : 0u;
 	atomicXor(ns + 2 * j, mine);
 	atomicXor(ns + 2 * j + 1, mine);
+}
+
+// The initial states of the lanes in `starting`, whose trajectories draw from `seed` and `stream` (fast mode: node
+// i's uniform is output i of the stream; all 32 lanes call it). The warp draws one lane's state at a time, a
+// Philox block a lane (about 300 instructions), or each starting lane draws its own (about 110 a block of four
+// nodes), whichever costs the warp less. 10 nodes, 1e6 trajectories
+// 0.91 -> 0.75 ms with the starts of eight lanes together.
+__device__ __forceinline__ void mb_lock_start(uint32_t* ns, mb_lock& v, unsigned long long seed, unsigned long long stream,
+											  const float* __restrict__ istate, bool starting)
+{
+	constexpr int blocks = (state_size + 3) / 4;
+	constexpr int own_cost = 110 * blocks + 6 * state_size, warp_cost = 300;
+	const int lane = threadIdx.x & 31;
+	unsigned pending = __ballot_sync(0xffffffffu, starting);
+	if (MB_LOCK_SMALL && __popc(pending) * warp_cost > own_cost)
+	{
+		if (starting)
+		{
+#pragma unroll
+			for (int w = 0; w < MB_LW; w++)
+			{
+				uint32_t bits = 0;
+#pragma unroll 1
+				for (int b = 8 * w; b < 8 * w + 8 && b < blocks; b++)
+				{
+					curandStatePhilox4_32_10_t r;
+					curand_init(seed, stream, 4ull * (unsigned long long)b, &r);
+					const float4 u = curand_uniform4(&r);
+					const int i = 4 * b;
+					uint32_t four = u.x <= __ldg(istate + i) ? 1u : 0u;
+					four |= i + 1 < state_size && u.y <= __ldg(istate + i + 1) ? 2u : 0u;
+					four |= i + 2 < state_size && u.z <= __ldg(istate + i + 2) ? 4u : 0u;
+					four |= i + 3 < state_size && u.w <= __ldg(istate + i + 3) ? 8u : 0u;
+					bits |= four << (4 * (b - 8 * w));
+				}
+				v.s[w] = bits;
+			}
+		}
+		return;
+	}
+	uint32_t* words = ns + 64 * MB_LW + 2; // (the gates' words)
+	while (pending)
+	{
+		const int src = __ffs(pending) - 1;
+		pending &= pending - 1u;
+		const unsigned long long from = __shfl_sync(0xffffffffu, stream, src);
+		const float* p = reinterpret_cast<const float*>(
+			__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(istate), src));
+		mb_philox_initial_state(seed, from, state_size, p, [&](int w, uint32_t word) {
+			if (lane == 0)
+				words[w] = word;
+		});
+		__syncwarp();
+		if (lane == src)
+		{
+#pragma unroll
+			for (int w = 0; w < MB_LW; w++)
+				v.s[w] = words[w];
+		}
+		__syncwarp();
+	}
 }
 
 // The nodes of word w whose rate may differ from the last step's: unstable then or now but not both, or the
@@ -1014,8 +1083,7 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_exact
 		if (!(idle | busy))
 			break;
 		bool starting = false;
-		// a warp waits for two lanes to start together while others run: the start's cost is the warp's (50
-		// nodes 5.73 -> 5.54 ms; with four 5.49, but the 87-node example model 3 % slower)
+		// a warp waits for two lanes to start together while others run: the start's cost is the warp's
 		if (working && !running && (__popc(idle) >= 2 || !busy))
 		{
 			const unsigned long long t = atomicAdd(P.next_traj, 1ull);
@@ -1327,9 +1395,7 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_fast(
 			break;
 		unsigned long long t = 0;
 		bool starting = false;
-		// a warp waits for two lanes to start together while others run: the start's cost is the warp's (50
-		// nodes 5.73 -> 5.54 ms; with four 5.49, but the 87-node example model 3 % slower)
-		if (working && !running && (__popc(idle) >= 2 || !busy))
+		if (working && !running && (__popc(idle) >= MB_LOCK_STARTS || !busy))
 		{
 			t = atomicAdd(P.next_traj, 1ull);
 			if (t < P.n_traj)
@@ -1337,28 +1403,9 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_fast(
 			else
 				working = false;
 		}
-		unsigned pending = __ballot_sync(0xffffffffu, starting);
-		if (pending)
+		if (__any_sync(0xffffffffu, starting))
 		{
-			uint32_t* words = ns + 64 * MB_LW + 2; // (the gates' words)
-			while (pending)
-			{
-				const int src = __ffs(pending) - 1;
-				pending &= pending - 1u;
-				const unsigned long long ts = __shfl_sync(0xffffffffu, t, src);
-				mb_philox_initial_state(P.seed, P.first_traj + ts, state_size, P.istate, [&](int w, uint32_t word) {
-					if (lane == 0)
-						words[w] = word;
-				});
-				__syncwarp();
-				if (lane == src)
-				{
-#pragma unroll
-					for (int w = 0; w < MB_LW; w++)
-						v.s[w] = words[w];
-				}
-				__syncwarp();
-			}
+			mb_lock_start(ns, v, P.seed, P.first_traj + t, P.istate, starting);
 			if (starting)
 			{
 				// after the N initial-state uniforms, every step uses one whole Philox block (4 x 32 bits)
