@@ -1117,9 +1117,10 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 		// per thread in shared memory: state words, unstable masks and word rate sums; or per warp its array
 		constexpr size_t max_smem = 227 * 1024;
 		block = std::min(block, 128);
-		if (m.table_threads && c.blocks_per_sm <= 0)
+		if (m.table_threads && c.blocks_per_sm <= 0 && c.block > 128)
 		{
-			// one block an SM with all that fits; in a small run only the warps that it needs on each SM
+			// (no shape of at most 128 threads asked for) one block an SM with all that fits; in a small run only
+			// the warps that it needs on each SM
 			const long long lanes = lanes_per_warp(n, m.ctx->sm_count), warps = (n + lanes - 1) / lanes;
 			block = (int)std::min<long long>(m.table_threads, 32 * ((warps + m.ctx->sm_count - 1) / m.ctx->sm_count));
 		}
