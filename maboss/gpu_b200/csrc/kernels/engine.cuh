@@ -6,7 +6,8 @@
 // Two execution shapes share the same per-step semantics (src/jit_kernels/simulation.cu:77-164):
 //  * fused persistent kernel: one thread runs whole trajectories taken from a work counter and
 //    accumulates window occupancy, transition entropy, final states and fixed points in place,
-//    so no trajectory buffer is written;
+//    so no trajectory buffer is written; in networks of at most 256 nodes the threads of a warp are in
+//    step and evaluate the logic of their 32 trajectories together (lockstep kernels);
 //  * buffered epoch kernels: the reference's simulate -> stats -> partition/refill epochs over
 //    SoA buffers [slot][word][trajectory], for the stats-plugin API.
 // Window sums are int64 fixed point (value * 2^e, round to nearest even): integer atomics make
@@ -1567,9 +1568,9 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_fast(
 	}
 }
 #else
-// at least 5 resident blocks of 128: 89 registers on the 1000-node network, no spills. Measured
-// (autotuned shapes): the 1000-node network runs equally at 4 and 5 (shared memory limits it to 3
-// or 4 blocks), the 50-node network 5.6 % faster at 5; at 6 the 1000-node network loses 11 %.
+// One block an SM with the tables in shared memory; networks whose tables leave fewer than 256 threads: at least 5
+// resident blocks of 128 (89 registers on the 1000-node network; with its tables in global memory it ran
+// equally at 4 and 5 and lost 11 % at 6).
 extern "C" __global__ void MB_FUSED_BOUNDS(128, 5) mb_fused_fast(mb_fused_params P)
 {
 	extern __shared__ __align__(16) uint32_t mb_smem_u32[];
