@@ -319,8 +319,31 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 	}
 	std::vector<mb_variant> hvars(vars_.size());
 	unsigned long long begin = 0;
-	size_t host_bytes = 0;
 	ps->host_off.resize(vars_.size());
+	bool fresh = false;
+	for (auto& vp : vars_)
+		fresh |= !vp->ready;
+	if (fresh)
+	{
+		// the arena is laid out anew for all variants (both kinds of run share it; the plans that hold the old
+		// addresses are gone: adding a variant drops them)
+		for (auto& vp : vars_)
+			if (!vp->ready)
+			{
+				const model_layout& L = nets[vp->net]->L;
+				vp->st.init_plain(L.state_words, L.time_tick, L.max_time, L.discrete_time, L.noninternal_nodes, vp->n_traj,
+								  vp->grad_params.size());
+			}
+		size_t front = 0, back = 0;
+		for (auto& vp : vars_)
+			vp->st.place(nullptr, front, back);
+		arena_front = (front + 255) / 256 * 256;
+		arena.alloc(arena_front + back);
+		size_t f = 0, b = arena_front;
+		for (auto& vp : vars_)
+			vp->st.place(static_cast<char*>(arena.p), f, b);
+		MB_CUDA(cudaMemsetAsync(arena.p, 0, arena.bytes, s));
+	}
 	for (size_t i = 0; i < vars_.size(); i++)
 	{
 		variant& V = *vars_[i];
@@ -330,11 +353,7 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 		if (!V.ready)
 		{
 			// created once: the other kind of run (forward / gradient) shares these buffers
-			V.st.init_plain(L.state_words, L.time_tick, L.max_time, L.discrete_time, L.noninternal_nodes, V.n_traj,
-							s);
 			upload(V.d_istate, V.istate, s);
-			V.d_counters.alloc(16);
-			V.d_grad.alloc(std::max<size_t>(1, V.grad_params.size()) * sizeof(double));
 			V.d_cot.alloc((size_t)L.windows() * ((size_t)1 << L.noninternal_nodes.size()) * sizeof(double));
 			V.out_states.alloc((size_t)V.st.fp_cap * L.state_words * 4);
 			V.out_counts.alloc((size_t)V.st.fp_cap * 4);
@@ -352,33 +371,28 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 		d.first_traj = V.first_traj;
 		d.n_traj = (unsigned)V.n_traj;
 		d.st = V.st.p;
-		d.transitions = V.d_counters.as<unsigned long long>();
+		d.transitions = V.st.transitions.as<unsigned long long>();
 		d.cot = grad ? V.d_cot.as<double>() : nullptr;
 		d.g_ptr = V.d_gptr.as<int>();
 		d.g_p = V.d_gp.as<int>();
 		d.g_d = V.d_gd.as<float>();
-		d.grad = V.d_grad.as<double>();
+		d.grad = V.st.grad.as<double>();
 		begin += (unsigned long long)V.n_traj;
-		// pinned host arena: windows, entropy sums, final counts, stats counters, transitions, gradient
+		// the pinned host copy has the arena's layout
+		auto off = [&](const dview& x) { return (size_t)(static_cast<char*>(x.p) - static_cast<char*>(arena.p)); };
 		host_off_t& o = ps->host_off[i];
-		o.win = host_bytes;
-		host_bytes += V.st.occ.bytes > 8 ? V.st.occ.bytes : V.st.cnt.bytes;
-		o.h = host_bytes;
-		host_bytes += V.st.h.bytes;
-		o.fin = host_bytes;
-		host_bytes += (V.st.fin.bytes + 7) / 8 * 8;
-		o.ctr = host_bytes;
-		host_bytes += 8;
-		o.trans = host_bytes;
-		host_bytes += 8;
-		o.grad = host_bytes;
-		host_bytes += V.d_grad.bytes;
+		o.win = off(V.st.win);
+		o.h = off(V.st.h);
+		o.fin = off(V.st.fin);
+		o.ctr = off(V.st.counters);
+		o.trans = off(V.st.transitions);
+		o.grad = off(V.st.grad);
 	}
 	upload(ps->d_nets, hnets, s);
 	upload(ps->d_vars, hvars, s);
 	ps->hvars = hvars;
 	ps->counters.alloc(64);
-	MB_CUDA(cudaHostAlloc(&ps->host, std::max<size_t>(host_bytes, 8), cudaHostAllocDefault));
+	MB_CUDA(cudaHostAlloc(&ps->host, std::max<size_t>(arena_front, 8), cudaHostAllocDefault));
 	MB_CUDA(cudaEventCreate(&ps->e0));
 	MB_CUDA(cudaEventCreate(&ps->e1));
 	ps->B = std::make_unique<mb_batch_params>();
@@ -474,13 +488,8 @@ void batch_engine::enqueue(prepared& ps, cudaStream_t s, bool capturing)
 		else
 			MB_CUDA(cudaEventRecord(e, s));
 	};
-	for (auto& vp : vars_)
-	{
-		variant& V = *vp;
-		V.st.zero(s);
-		MB_CUDA(cudaMemsetAsync(V.d_counters.p, 0, V.d_counters.bytes, s));
-		MB_CUDA(cudaMemsetAsync(V.d_grad.p, 0, V.d_grad.bytes, s));
-	}
+	if (arena.p)
+		MB_CUDA(cudaMemsetAsync(arena.p, 0, arena.bytes, s));
 	MB_CUDA(cudaMemsetAsync(ps.counters.p, 0, ps.counters.bytes, s));
 	record(ps.e0);
 	if (ps.B->total > 0)
@@ -500,20 +509,10 @@ void batch_engine::enqueue(prepared& ps, cudaStream_t s, bool capturing)
 		}
 	}
 	record(ps.e1);
-	char* host = static_cast<char*>(ps.host);
-	for (size_t i = 0; i < vars_.size(); i++)
-	{
-		variant& V = *vars_[i];
-		const host_off_t& o = ps.host_off[i];
-		V.st.extract(s, V.out_states.as<unsigned>(), V.out_counts.as<unsigned>(), print6(nets[V.net]->L.max_time));
-		dbuf& win = V.st.occ.bytes > 8 ? V.st.occ : V.st.cnt;
-		MB_CUDA(cudaMemcpyAsync(host + o.win, win.p, win.bytes, cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(host + o.h, V.st.h.p, V.st.h.bytes, cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(host + o.fin, V.st.fin.p, V.st.fin.bytes, cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(host + o.ctr, V.st.counters.p, 8, cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(host + o.trans, V.d_counters.p, 8, cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(host + o.grad, V.d_grad.p, V.d_grad.bytes, cudaMemcpyDeviceToHost, s));
-	}
+	for (auto& vp : vars_)
+		vp->st.extract(s, vp->out_states.as<unsigned>(), vp->out_counts.as<unsigned>(), print6(nets[vp->net]->L.max_time));
+	if (arena_front)
+		MB_CUDA(cudaMemcpyAsync(ps.host, arena.p, arena_front, cudaMemcpyDeviceToHost, s));
 }
 
 // Times the candidate launch shapes on the batch itself (one run each after a warm-up run) and keeps
@@ -647,7 +646,7 @@ void batch_engine::run(unsigned long long seed, const std::vector<std::vector<do
 // ---- per-variant accumulators (same layout and fixed-point scales as stats_state)
 
 void plain_stats::init_plain(int words, float tick, float tmax, bool discrete, const std::vector<int>& noninternal,
-							 long long n, cudaStream_t s)
+							 long long n, size_t n_grad)
 {
 	W = words;
 	const int k = (int)noninternal.size();
@@ -661,47 +660,49 @@ void plain_stats::init_plain(int words, float tick, float tmax, bool discrete, c
 	fx = std::ldexp(1.0, occupancy_exponent(n, tick, discrete));
 	fx_h = std::ldexp(1.0, entropy_exponent(n, tick, discrete));
 	const size_t cells = (size_t)n_windows * n_bins;
-	occ.alloc(discrete ? 8 : cells * sizeof(long long));
-	if (!discrete && cells <= tail_max_cells)
-	{
-		tail.alloc(cells * sizeof(unsigned));
-		MB_CUDA(cudaMemsetAsync(tail.p, 0, tail.bytes, s)); // (each run leaves it cleared)
-	}
-	cnt.alloc(discrete ? cells * sizeof(unsigned) : 4);
-	h.alloc(n_windows * sizeof(long long));
-	fin.alloc(n_bins * sizeof(unsigned));
 	unsigned cap = 1024;
 	while (cap < 2 * std::min<long long>(std::max(n, 1LL), 1LL << 22))
 		cap <<= 1;
 	fp_cap = cap;
-	fp_keys.alloc((size_t)cap * sizeof(mb_key128));
-	fp_counts.alloc((size_t)cap * sizeof(unsigned));
 	fp_states.alloc((size_t)cap * W * sizeof(unsigned));
-	counters.alloc(64);
-	zero(s);
+	counters.bytes = 64;
+	transitions.bytes = 16;
+	grad.bytes = std::max<size_t>(1, n_grad) * sizeof(double);
+	h.bytes = n_windows * sizeof(long long);
+	fin.bytes = n_bins * sizeof(unsigned);
+	win.bytes = cells * (discrete ? sizeof(unsigned) : sizeof(long long));
+	tail.bytes = !discrete && cells <= tail_max_cells ? cells * sizeof(unsigned) : 0;
+	fp_keys.bytes = (size_t)cap * sizeof(mb_key128);
+	fp_counts.bytes = (size_t)cap * sizeof(unsigned);
+}
+
+void plain_stats::place(char* arena, size_t& front, size_t& back)
+{
+	auto put = [&](dview& v, size_t& at) {
+		v.p = arena && v.bytes ? arena + at : nullptr;
+		at += (v.bytes + 63) / 64 * 64;
+	};
+	for (dview* v : { &counters, &transitions, &grad, &h, &fin, &win })
+		put(*v, front);
+	for (dview* v : { &tail, &fp_keys, &fp_counts })
+		put(*v, back);
 	p = mb_stats_params{};
 	p.n_windows = n_windows;
 	p.n_bins = n_bins;
-	p.win_tick = tick;
+	p.win_tick = time_tick;
 	p.h_in_smem = 0;
 	p.fx = fx;
 	p.fx_h = fx_h;
-	p.win_occ = occ.as<long long>();
-	p.win_cnt = cnt.as<unsigned>();
+	p.win_occ = discrete_time ? nullptr : win.as<long long>();
+	p.win_cnt = discrete_time ? win.as<unsigned>() : nullptr;
 	p.win_h = h.as<long long>();
 	p.final_cnt = fin.as<unsigned>();
 	p.fp_keys = fp_keys.as<mb_key128>();
 	p.fp_counts = fp_counts.as<unsigned>();
 	p.fp_states = fp_states.as<unsigned>();
-	p.fp_mask = cap - 1;
+	p.fp_mask = fp_cap - 1;
 	p.fp_overflow = counters.as<unsigned>();
 	p.tail = tail.as<unsigned>();
-}
-
-void plain_stats::zero(cudaStream_t s)
-{
-	for (dbuf* b : { &occ, &cnt, &h, &fin, &fp_keys, &fp_counts, &counters })
-		MB_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, s));
 }
 
 void plain_stats::extract(cudaStream_t s, unsigned* out_states, unsigned* out_counts, float sim_max_time)

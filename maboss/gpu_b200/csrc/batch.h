@@ -19,7 +19,10 @@ namespace mb {
 // compiled module).
 struct plain_stats
 {
-	dbuf occ, cnt, h, fin, fp_keys, fp_counts, fp_states, counters, tail;
+	// parts of the batch's arena: the front is copied back by every run, all of it is cleared
+	dview counters, transitions, grad, h, fin, win; // win: occupancy (continuous) or counts (discrete)
+	dview tail, fp_keys, fp_counts;
+	dbuf fp_states;
 	unsigned fp_cap = 0;
 	int W = 1, n_windows = 0;
 	unsigned n_bins = 0;
@@ -29,8 +32,10 @@ struct plain_stats
 	std::vector<int> noninternal_nodes;
 	mb_stats_params p{};
 	void init_plain(int words, float tick, float tmax, bool discrete, const std::vector<int>& noninternal, long long n,
-					cudaStream_t s);
-	void zero(cudaStream_t s); // clear every accumulator (asynchronous, capturable)
+					size_t n_grad);
+	// puts the accumulators at the arena's offsets `front` and `back`, which move behind them (with a null
+	// arena: only the offsets)
+	void place(char* arena, size_t& front, size_t& back);
 	// compact the fixed-point table into (state, count) records; their number goes to counters[1]
 	// (and add the window sums of the trajectories counted at their fixed point; `sim_max_time` is the
 	// generated code's max_time)
@@ -65,7 +70,7 @@ public:
 		int rate_shift = 0;
 		std::vector<unsigned> q;
 		plain_stats st;
-		dbuf d_q, d_rate, d_rlog, d_istate, d_gptr, d_gp, d_gd, d_counters, d_grad, d_cot, out_states, out_counts;
+		dbuf d_q, d_rate, d_rlog, d_istate, d_gptr, d_gp, d_gd, d_cot, out_states, out_counts;
 		bool ready = false; // accumulators and per-variant buffers exist (created once, shared by both plans)
 		std::unique_ptr<result> res;
 		std::vector<double> grad; // d (sum_ws cot[w][s] P_w(s)) / d parameter
@@ -107,6 +112,10 @@ public:
 	float kernel_ms = 0;
 	int last_block = 0, last_per_sm = 0;
 	unsigned last_grid = 0;
+	// every variant's accumulators: the fronts, then the backs (one clear and one copy a run for all variants, not
+	// nine clears and six copies for each)
+	dbuf arena;
+	size_t arena_front = 0;
 	unsigned graph_nodes = 0; // nodes of the last captured graph
 
 private:
