@@ -493,7 +493,10 @@ void module::ensure(int family)
 		{
 			const std::vector<unsigned>& t = xorwow_jump_table();
 			dbuf b(t.size() * sizeof(unsigned));
-			MB_CUDA(cudaMemcpy(b.p, t.data(), b.bytes, cudaMemcpyHostToDevice));
+			// on the context's stream and waited for: cudaMemcpy may return before a copy from pageable memory has
+			// reached the device, and neither that stream (non-blocking) nor a caller's waits for the default one
+			MB_CUDA(cudaMemcpyAsync(b.p, t.data(), b.bytes, cudaMemcpyHostToDevice, ctx->stream));
+			MB_CUDA(cudaStreamSynchronize(ctx->stream));
 			ctx->xorwow_jump = std::move(b);
 		}
 		get(init_random, "mb_initialize_random");
