@@ -356,7 +356,7 @@ module::~module()
 		if (e)
 			cudaEventDestroy(e);
 	for (int f = 0; f < FAMILY_COUNT; f++)
-		if (mods[f] && f != FAMILY_BATCH)
+		if (mods[f])
 			drv().ModuleUnload(mods[f]);
 	if (batch_lib)
 		cudaLibraryUnload(batch_lib);
@@ -455,30 +455,38 @@ std::mutex family_mu;
 void module::ensure(int family)
 {
 	std::lock_guard<std::mutex> lk(family_mu);
-	if (mods[family])
+	if (loaded[family])
 		return;
 	MB_CUDA(cudaSetDevice(ctx->device));
-	auto t0 = std::chrono::steady_clock::now();
-	std::string lg;
-	std::vector<char> cubin = compile_cubin(source, lg, family);
-	compile_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-	if (!lg.empty())
-		log += lg;
-	if (family == FAMILY_BATCH)
+	if (!mods[family])
 	{
-		cudaKernel_t kf = nullptr, kg = nullptr;
-		MB_CUDA(cudaLibraryLoadData(&batch_lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-		MB_CUDA(cudaLibraryGetKernel(&kf, batch_lib, "mb_batched_fast_static"));
-		MB_CUDA(cudaLibraryGetKernel(&kg, batch_lib, "mb_batched_grad_static"));
-		batched_fast_static = reinterpret_cast<const void*>(kf);
-		batched_grad_static = reinterpret_cast<const void*>(kg);
-		mods[family] = reinterpret_cast<CUmodule>(batch_lib); // marks the family as loaded
-		return;
+		auto t0 = std::chrono::steady_clock::now();
+		std::string lg;
+		std::vector<char> cubin = compile_cubin(source, lg, family);
+		compile_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+		if (!lg.empty())
+			log += lg;
+		if (family == FAMILY_BATCH)
+		{
+			cudaKernel_t kf = nullptr, kg = nullptr;
+			if (!batch_lib)
+				MB_CUDA(cudaLibraryLoadData(&batch_lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+			MB_CUDA(cudaLibraryGetKernel(&kf, batch_lib, "mb_batched_fast_static"));
+			MB_CUDA(cudaLibraryGetKernel(&kg, batch_lib, "mb_batched_grad_static"));
+			batched_fast_static = reinterpret_cast<const void*>(kf);
+			batched_grad_static = reinterpret_cast<const void*>(kg);
+			loaded[family] = true;
+			return;
+		}
+		CUmodule cm = nullptr;
+		cu_throw(drv().ModuleLoadData(&cm, cubin.data()), "cuModuleLoadData");
+		mods[family] = cm;
 	}
-	CUmodule cm = nullptr;
-	cu_throw(drv().ModuleLoadData(&cm, cubin.data()), "cuModuleLoadData");
-	mods[family] = cm;
-	auto get = [&](CUfunction& f, const char* name) { cu_throw(drv().ModuleGetFunction(&f, cm, name), name); };
+	// a call that fails below leaves the family not loaded: the next one goes on with the module that is there
+	// (init_random and init_state mark their groups, so they are set last)
+	auto get = [&](CUfunction& f, const char* name) {
+		cu_throw(drv().ModuleGetFunction(&f, mods[family], name), name);
+	};
 	if (family == FAMILY_EXACT)
 		get(fused_exact, "mb_fused_exact");
 	if (family == FAMILY_FAST)
@@ -503,7 +511,6 @@ void module::ensure(int family)
 	}
 	if (!init_state)
 	{
-		get(init_state, "mb_initialize_initial_state");
 		get(window_epoch, "mb_window_epoch");
 		get(final_epoch, "mb_final_epoch");
 		get(fixed_epoch, "mb_fixed_epoch");
@@ -512,7 +519,9 @@ void module::ensure(int family)
 		get(compact_scatter, "mb_compact_scatter");
 		get(fixed_extract, "mb_fixed_extract");
 		get(bins_extract, "mb_bins_extract");
+		get(init_state, "mb_initialize_initial_state");
 	}
+	loaded[family] = true;
 }
 
 void module::ensure_any()

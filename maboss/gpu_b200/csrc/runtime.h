@@ -166,6 +166,7 @@ struct module
 {
 	context* ctx = nullptr;
 	CUmodule mods[FAMILY_COUNT] = { nullptr, nullptr, nullptr, nullptr, nullptr };
+	bool loaded[FAMILY_COUNT] = { false, false, false, false, false }; // with every handle and table its kernels need
 	// FAMILY_BATCH is loaded as a runtime-API library: its kernels are cudaKernel_t handles, which the
 	// batch engine's runtime-API launches, occupancy queries and graph nodes take like its own kernels
 	cudaLibrary_t batch_lib = nullptr;

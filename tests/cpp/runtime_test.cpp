@@ -92,12 +92,37 @@ void jump_table_is_there_before_the_first_launch()
 	}
 }
 
+// A family that could not be loaded whole is not taken for loaded: the next call loads the rest.
+void family_loads_after_a_failure()
+{
+	{
+		program p;
+		bool fail = true;
+		fake::fail_malloc = [&](size_t) { return fail; };
+		CHECK(throws([&] { p.m->ensure(mb::FAMILY_EXACT); }));
+		fail = false;
+		p.m->ensure(mb::FAMILY_EXACT);
+		CHECK(p.m->fused_exact && p.m->init_random && p.ctx.xorwow_jump.p);
+		fake::fail_malloc = nullptr;
+	}
+	for (const char* name : { "mb_simulate_epoch", "mb_initialize_random" })
+	{
+		program p;
+		fake::fail_function = name;
+		CHECK(throws([&] { p.m->ensure(mb::FAMILY_EPOCH); }));
+		fake::fail_function.clear();
+		p.m->ensure(mb::FAMILY_EPOCH);
+		CHECK(p.m->sim_epoch && p.m->init_random);
+	}
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
 	const std::map<std::string, void (*)()> checks = {
 		{ "jump_table_is_there_before_the_first_launch", jump_table_is_there_before_the_first_launch },
+		{ "family_loads_after_a_failure", family_loads_after_a_failure },
 	};
 	for (int i = 1; i < argc; i++)
 		checks.at(argv[i])();
