@@ -842,7 +842,8 @@ __device__ __forceinline__ float mb_exact_entropy(const V& v)
 }
 
 // select_flip_bit: the first node whose running fp32 sum reaches r; its word is the first whose
-// word-end sum reaches r (r <= total = the last word-end sum).
+// word-end sum reaches r (r <= total = the last word-end sum). Node 0 where r is 0, the product of a very
+// small total and a uniform number, whether or not it is unstable: every sum reaches 0.
 template <class V>
 __device__ __forceinline__ int mb_exact_select(const V& v, float r)
 {
@@ -856,9 +857,9 @@ __device__ __forceinline__ int mb_exact_select(const V& v, float r)
 			wh = mid;
 	}
 	float sum = wl > 0 ? __uint_as_float(v.Q(wl - 1)) : 0.f;
-	uint32_t um = v.U(wl);
+	uint32_t um = r > 0.f ? v.U(wl) : 0u;
 	const uint32_t sw = v.S(wl);
-	int j = -1;
+	int j = 0;
 	while (um)
 	{
 		const int b = __ffs(um) - 1;
@@ -993,10 +994,10 @@ __device__ __forceinline__ int mb_lock_exact_select(const mb_lock& v, const floa
 		word += lt ? 1 : 0;
 		sum = lt ? q[w] : sum;
 	}
-	uint32_t um = v.pick(v.u, word);
+	uint32_t um = r > 0.f ? v.pick(v.u, word) : 0u;
 	const uint32_t sw = v.pick(v.s, word);
 	const float* rate = mbg_inc_rate + 64 * word;
-	int j = -1;
+	int j = 0;
 	while (um)
 	{
 		const int b0 = __ffs(um) - 1;
