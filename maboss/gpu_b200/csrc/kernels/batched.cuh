@@ -529,7 +529,7 @@ __device__ void mbb_body(const mb_batch_params& B)
 				mb_fixed_insert_rt(var.st, st, W);
 				if (GRAD)
 					mbb_grad_end(v, P, discrete, C1, C2);
-				atomicAdd(var.transitions, trans + 1);
+				atomicAdd(var.transitions, trans + (max_time != 0.f ? 1 : 0)); // (steps that end at time 0 are empty)
 				trans = 0;
 				break;
 			}
@@ -892,7 +892,7 @@ __device__ void mbb_lock_body(const mb_batch_params& B)
 					st[w] = v.s[w];
 				mb_fixed_insert_rt(var.st, st, MB_LW);
 				ended = true;
-				atomicAdd(var.transitions, trans + 1);
+				atomicAdd(var.transitions, trans + (end_time != 0.f ? 1 : 0));
 				trans = 0;
 			}
 			else

@@ -119,6 +119,20 @@ __device__ __forceinline__ void mb_record(mb_win_acc& a, const mb_stats_params& 
 		mb_record_cont(a, p, hsink, idx, t0, t1, h);
 }
 
+// The last step of a trajectory at a fixed point that it reached at t0: its state stays until max_time. Returns
+// the transitions counted for it: one, or none where max_time is 0 (steps that end at time 0 are empty).
+__device__ __forceinline__ unsigned mb_record_stay(mb_win_acc& a, const mb_stats_params& p, long long* hsink, mb_idx_t idx,
+												   float t0, unsigned* counts = nullptr)
+{
+	if (max_time == 0.f)
+		return 0u;
+	if (discrete_time)
+		mb_record_disc(p, hsink, idx, t0, 0.f, counts);
+	else
+		mb_record_fixed(a, p, hsink, idx, t0, max_time);
+	return 1u;
+}
+
 // ---------------------------------------------------------------- fused persistent kernel
 
 // One whole trajectory. EXACT reproduces the reference bit for bit: XORWOW streams seeded by
@@ -1129,11 +1143,7 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_exact
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				trans++;
-				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, 0.f, counts);
-				else
-					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				trans += mb_record_stay(acc, P.st, hsink, idx, time, counts);
 				mb_final_add(P.st, idx);
 				mb_fixed_insert(P.st, v.s);
 			}
@@ -1277,11 +1287,7 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_param
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				trans++;
-				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, 0.f);
-				else
-					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				trans += mb_record_stay(acc, P.st, hsink, idx, time);
 				mb_final_add(P.st, idx);
 				state_word_t st[state_words];
 #pragma unroll
@@ -1461,11 +1467,7 @@ extern "C" __global__ void __launch_bounds__(128, MB_LOCK_BLOCKS) mb_fused_fast(
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				trans++;
-				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, 0.f, counts);
-				else
-					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				trans += mb_record_stay(acc, P.st, hsink, idx, time, counts);
 				mb_final_add(P.st, idx);
 				mb_fixed_insert(P.st, v.s);
 			}
@@ -1654,11 +1656,7 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 5) mb_fused_fast(mb_fused_params
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
-				trans++;
-				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, 0.f);
-				else
-					mb_record_fixed(acc, P.st, hsink, idx, time, max_time);
+				trans += mb_record_stay(acc, P.st, hsink, idx, time);
 				mb_final_add(P.st, idx);
 				state_word_t st[state_words];
 #pragma unroll
