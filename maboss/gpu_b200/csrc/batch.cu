@@ -25,6 +25,8 @@ namespace mb {
 
 namespace {
 
+constexpr size_t max_smem = 227 * 1024; // of a block
+
 // compaction of one variant's fixed-point table into (state, count) records; the first `tail_blocks`
 // blocks add the window sums of the trajectories that mb_record_fixed counted
 __global__ void __launch_bounds__(32 * MB_TAIL_COLS) mbb_fixed_extract(mb_stats_params p, float max_time,
@@ -417,16 +419,30 @@ batch_engine::prepared& batch_engine::prepare(bool grad)
 		if (N.mod->gate_words && vars_.size() == 1 && vars_[0]->st.n_windows <= 1024)
 			B.h_windows = vars_[0]->st.n_windows;
 	}
+	ps->rows_per_thread = (3 * (size_t)max_W + (grad ? 2 * (size_t)P : 0)) * 4;
 	ps->smem_per_thread = ((ps->smem_per_warp ? 0 : 3 * (size_t)max_W) + (grad ? 2 * (size_t)P : 0)) * 4;
 	MB_CUDA(cudaStreamSynchronize(s));
 	slot = std::move(ps);
 	return *slot;
 }
 
+// The most threads, up to `block`, that the plan's kernel runs with where the general kernel runs with `block`.
+// A lockstep kernel's arrays and entropy sums can be larger than the rows that they replace (many gates, or
+// many windows: 20 nodes, 1000 windows and 220 parameters take 128 threads 226,816 bytes of rows, but 234,848),
+// so a batch that just fits as rows runs with fewer threads. 0: too large for either.
+int batch_engine::largest_block(prepared& ps, int block) const
+{
+	if ((size_t)block * ps.rows_per_thread > max_smem)
+		return 0;
+	size_t smem = 0;
+	while (block >= 32 && fit(ps, block, smem) < 1)
+		block -= 32;
+	return block;
+}
+
 // Blocks per SM that fit a launch shape, and the shared memory of a block.
 int batch_engine::fit(prepared& ps, int block, size_t& smem) const
 {
-	constexpr size_t max_smem = 227 * 1024;
 	smem = (size_t)block * ps.smem_per_thread + (size_t)(block / 32) * ps.smem_per_warp + (size_t)ps.B->h_windows * sizeof(long long);
 	if (smem > max_smem)
 		return 0;
@@ -530,6 +546,8 @@ void batch_engine::tune(prepared& ps, cudaStream_t s)
 		if (per_sm >= 2)
 			cands.push_back({ block, per_sm - 1 });
 	}
+	if (cands.empty() && largest_block(ps, 64) > 0)
+		cands.push_back({ largest_block(ps, 64), 0 });
 	if (cands.empty())
 		throw engine_error(MB_ERR_LIMIT, "batch too large for shared memory (state words, gradient parameters)");
 	float best = 0.f;
@@ -577,7 +595,10 @@ void batch_engine::run(unsigned long long seed, const std::vector<std::vector<do
 		if (autotune && ps.B->total > 0)
 			tune(ps, s);
 		else
-			set_shape(ps, 128, 0);
+		{
+			const int block = largest_block(ps, 128);
+			set_shape(ps, block > 0 ? block : 128, 0);
+		}
 	}
 	if (use_graph)
 	{

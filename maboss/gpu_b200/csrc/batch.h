@@ -130,6 +130,7 @@ private:
 		const void* fn = nullptr;
 		size_t smem_per_warp = 0; // the lockstep kernels' arrays
 		size_t smem_per_thread = 0, smem = 0;
+		size_t rows_per_thread = 0; // of the general kernels: what sets the limits of a batch
 		int block = 0, per_sm = 0;
 		unsigned grid = 0;
 		dbuf counters, gscratch;
@@ -148,6 +149,7 @@ private:
 	std::unique_ptr<prepared> prep[2]; // forward, gradient
 	void invalidate();
 	prepared& prepare(bool grad);
+	int largest_block(prepared& ps, int block) const;
 	int fit(prepared& ps, int block, size_t& smem) const;
 	void compute_rates(variant& V) const;
 	void upload_tables(variant& V, cudaStream_t s);
