@@ -658,6 +658,10 @@ model_layout analyze_model(const model_t& m)
 			if (mi > max_inputs || wide_patterns > (1LL << 18))
 				L.incremental_ok = false;
 		}
+		// (the dense kernels, which such logics had before, need no rows: a warp's and the entropy sums have to fit)
+		const size_t h = L.windows() <= 6144 ? (size_t)std::max(0, L.windows()) * 8 : 0;
+		if (L.max_inputs > incremental_record_inputs && (size_t)L.state_words * 384 + h > 227 * 1024)
+			L.incremental_ok = false;
 		if (L.incremental_ok)
 		{
 			L.in_ptr.push_back(0);
