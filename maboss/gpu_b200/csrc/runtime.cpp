@@ -20,6 +20,8 @@
 #include <sstream>
 #include <thread>
 
+#include <sys/mman.h>
+
 #include "kernels/params.cuh"
 
 namespace mb {
@@ -222,7 +224,7 @@ namespace {
 struct stage_pool
 {
 	std::mutex mu;
-	std::vector<std::pair<size_t, void*>> blocks;
+	std::vector<host_stage::block> blocks;
 	size_t kept = 0;
 	static constexpr size_t most = 64ull << 20;
 };
@@ -231,52 +233,119 @@ stage_pool& stages()
 	static stage_pool* pool = new stage_pool;
 	return *pool;
 }
+
+constexpr size_t huge_page = 2ull << 20;
+
+// Pinned memory, null where that fails. From 2 MB on it is mapped as huge pages and registered: 16 MB take 2
+// ms and 64 MB 8 ms, where cudaHostAlloc (4 KB pages) takes 9 and 24 ms, and a copy into new pageable memory
+// 7 and 29 ms. Below, cudaHostAlloc.
+host_stage::block pinned_block(size_t bytes)
+{
+	host_stage::block b;
+	b.size = bytes;
+	if (bytes < huge_page)
+	{
+		if (cudaHostAlloc(&b.p, bytes, cudaHostAllocPortable) != cudaSuccess)
+			b.p = nullptr;
+	}
+	else
+	{
+		b.mapped = bytes + huge_page; // room for the alignment
+		void* base = mmap(nullptr, b.mapped, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+		if (base != MAP_FAILED)
+		{
+			b.base = base;
+			b.p = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(base) + huge_page - 1) / huge_page * huge_page);
+			madvise(b.p, bytes, MADV_HUGEPAGE);
+			madvise(b.p, bytes, MADV_DONTFORK); // (a child that writes must not move the pages that are registered)
+			if (cudaHostRegister(b.p, bytes, cudaHostRegisterPortable) != cudaSuccess)
+			{
+				munmap(base, b.mapped);
+				b.p = nullptr;
+			}
+		}
+	}
+	if (!b.p)
+		(void)cudaGetLastError();
+	return b;
+}
+
+void free_block(const host_stage::block& b) noexcept
+{
+	if (b.mapped)
+	{
+		cudaHostUnregister(b.p);
+		munmap(b.base, b.mapped);
+	}
+	else
+		cudaFreeHost(b.p);
+}
 } // namespace
 
 void host_stage::reserve(size_t bytes)
 {
-	if (bytes <= size)
+	if (bytes <= b.size)
 		return;
 	release();
+	// powers of two below 2 MB, above whole huge pages with an eighth to spare (the next run's lists differ a little)
 	size_t want = 4096;
-	while (want < bytes)
-		want <<= 1;
+	if (bytes > huge_page / 2)
+		want = (bytes + bytes / 8 + huge_page - 1) / huge_page * huge_page;
+	else
+		while (want < bytes)
+			want <<= 1;
+	stage_pool& pool = stages();
+	{
+		// the smallest block that holds them, of at most four times the size or 8 MB
+		std::lock_guard<std::mutex> lk(pool.mu);
+		size_t best = pool.blocks.size();
+		for (size_t i = 0; i < pool.blocks.size(); i++)
+			if (pool.blocks[i].size >= bytes && pool.blocks[i].size <= std::max(4 * want, 4 * huge_page) &&
+				(best == pool.blocks.size() || pool.blocks[i].size <= pool.blocks[best].size))
+				best = i;
+		if (best < pool.blocks.size())
+		{
+			b = pool.blocks[best];
+			pool.blocks.erase(pool.blocks.begin() + (std::ptrdiff_t)best);
+			pool.kept -= b.size;
+			return;
+		}
+	}
+	b = pinned_block(want);
+	if (!b.p)
+	{
+		b = block();
+		b.p = std::malloc(want);
+		if (!b.p)
+			throw engine_error(MB_ERR_LIMIT, "out of host memory for the result's copies");
+		b.size = want;
+		b.pinned = false;
+	}
+}
+
+void host_stage::warm()
+{
 	stage_pool& pool = stages();
 	{
 		std::lock_guard<std::mutex> lk(pool.mu);
-		for (size_t i = pool.blocks.size(); i-- > 0;)
-			if (pool.blocks[i].first == want)
-			{
-				p = pool.blocks[i].second;
-				pool.blocks.erase(pool.blocks.begin() + (std::ptrdiff_t)i);
-				pool.kept -= want;
-				size = want;
-				pinned = true;
-				return;
-			}
+		if (!pool.blocks.empty())
+			return;
 	}
-	pinned = cudaHostAlloc(&p, want, cudaHostAllocPortable) == cudaSuccess;
-	if (!pinned)
-	{
-		(void)cudaGetLastError();
-		p = std::malloc(want);
-		if (!p)
-			throw engine_error(MB_ERR_LIMIT, "out of host memory for the result's copies");
-	}
-	size = want;
+	host_stage s;
+	s.reserve(2 * huge_page - 2 * huge_page / 8);
 }
 
 void host_stage::release() noexcept
 {
-	if (!p)
+	if (!b.p)
 		return;
-	std::vector<void*> freed;
-	if (!pinned)
-		std::free(p);
+	std::vector<block> freed;
+	if (!b.pinned)
+		std::free(b.p);
 	else
 	{
 		stage_pool& pool = stages();
-		bool keep = size <= stage_pool::most;
+		bool keep = b.size <= stage_pool::most;
 		{
 			std::lock_guard<std::mutex> lk(pool.mu);
 			try
@@ -284,8 +353,8 @@ void host_stage::release() noexcept
 				if (keep)
 				{
 					freed.reserve(pool.blocks.size());
-					pool.blocks.emplace_back(size, p);
-					pool.kept += size;
+					pool.blocks.push_back(b);
+					pool.kept += b.size;
 				}
 			}
 			catch (...)
@@ -294,18 +363,17 @@ void host_stage::release() noexcept
 			}
 			while (pool.kept > stage_pool::most) // (the block just returned is the last, and fits alone)
 			{
-				freed.push_back(pool.blocks.front().second);
-				pool.kept -= pool.blocks.front().first;
+				freed.push_back(pool.blocks.front());
+				pool.kept -= pool.blocks.front().size;
 				pool.blocks.erase(pool.blocks.begin());
 			}
 		}
 		if (!keep)
-			cudaFreeHost(p);
-		for (void* q : freed)
-			cudaFreeHost(q);
+			free_block(b);
+		for (const block& x : freed)
+			free_block(x);
 	}
-	p = nullptr;
-	size = 0;
+	b = block();
 }
 
 void dbuf::alloc(size_t n)
@@ -337,6 +405,7 @@ context::context(int dev) : device(dev)
 		throw engine_error(MB_ERR_NO_DEVICE, std::string("this engine is built for sm_100a (B200); device is ") +
 												 prop.name + " sm_" + std::to_string(cc_major) + std::to_string(cc_minor));
 	MB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+	host_stage::warm(); // 1 ms here, where making the context takes 900, so that small runs' first calls have it
 }
 
 context::~context()
@@ -844,16 +913,16 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 		MB_CUDA(cudaMemcpyAsync(&ovf, bin_overflow_ctr(), sizeof ovf, cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaStreamSynchronize(s));
 		// sorted on the device, copied into pinned memory, decoded by host threads
-		stage_keys.reserve((size_t)nb * sizeof(mb_key128));
-		stage_vals.reserve((size_t)nb * sizeof(long long));
+		stage.reserve((size_t)nb * (sizeof(mb_key128) + sizeof(long long)));
+		const size_t at_vals = (size_t)nb * sizeof(mb_key128);
 		if (nb)
 		{
 			sort_bins(ok, ov, nb, scratch, s);
-			MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), scratch.out_keys.p, nb * sizeof(mb_key128), cudaMemcpyDeviceToHost, s));
-			MB_CUDA(cudaMemcpyAsync(stage_vals.as<void>(), scratch.out_vals.p, nb * sizeof(long long), cudaMemcpyDeviceToHost, s));
+			MB_CUDA(cudaMemcpyAsync(stage.as<void>(), scratch.out_keys.p, nb * sizeof(mb_key128), cudaMemcpyDeviceToHost, s));
+			MB_CUDA(cudaMemcpyAsync(stage.as<void>(at_vals), scratch.out_vals.p, nb * sizeof(long long), cudaMemcpyDeviceToHost, s));
 			MB_CUDA(cudaStreamSynchronize(s));
 		}
-		decode_sorted_bins(stage_keys.as<uint64_t>(), stage_vals.as<long long>(), nb, n_windows, (int)std::thread::hardware_concurrency(),
+		decode_sorted_bins(stage.as<uint64_t>(), stage.as<long long>(at_vals), nb, n_windows, (int)std::thread::hardware_concurrency(),
 						   r.sp_w, r.sp_idx, r.sp_val, r.sp_begin, r.fin_idx, r.fin_cnt);
 		scratch.trim();
 		r.bin_overflow = ovf;
@@ -867,18 +936,18 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 										   cell_vals, m.ctx->sm_count, scratch, s);
 		if (nz >= 0)
 		{
-			stage_keys.reserve((size_t)nz * sizeof(unsigned long long));
-			stage_vals.reserve((size_t)nz * sizeof(long long));
+			stage.reserve((size_t)nz * (sizeof(unsigned long long) + sizeof(long long)));
+			const size_t at_vals = (size_t)nz * sizeof(unsigned long long);
 			if (nz)
 			{
-				MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), cell_idx.p, (size_t)nz * sizeof(unsigned long long),
+				MB_CUDA(cudaMemcpyAsync(stage.as<void>(), cell_idx.p, (size_t)nz * sizeof(unsigned long long),
 										cudaMemcpyDeviceToHost, s));
-				MB_CUDA(cudaMemcpyAsync(stage_vals.as<void>(), cell_vals.p, (size_t)nz * sizeof(long long),
+				MB_CUDA(cudaMemcpyAsync(stage.as<void>(at_vals), cell_vals.p, (size_t)nz * sizeof(long long),
 										cudaMemcpyDeviceToHost, s));
 				MB_CUDA(cudaStreamSynchronize(s));
 			}
-			const unsigned long long* idx = stage_keys.as<unsigned long long>();
-			const long long* vals = stage_vals.as<long long>();
+			const unsigned long long* idx = stage.as<unsigned long long>();
+			const long long* vals = stage.as<long long>(at_vals);
 			r.sp_w.resize((size_t)nz);
 			r.sp_idx.resize((size_t)nz);
 			r.sp_val.resize((size_t)nz);
@@ -890,6 +959,8 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 					r.sp_val[i] = vals[i];
 				}
 			});
+			if (stage.bytes() > max_kept_stage)
+				stage.release();
 			r.sp_begin.assign((size_t)n_windows + 1, 0);
 			for (int w = 0; w <= n_windows; w++)
 				r.sp_begin[w] = (size_t)(std::lower_bound(r.sp_w.begin(), r.sp_w.end(), w) - r.sp_w.begin());
@@ -947,12 +1018,12 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 	std::vector<unsigned> st((size_t)nfp * W), cn(nfp);
 	if (nfp > first)
 	{
-		stage_keys.reserve((size_t)nfp * (W + 1) * sizeof(unsigned));
-		MB_CUDA(cudaMemcpyAsync(stage_keys.as<void>(), out_counts.p, nfp * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-		MB_CUDA(cudaMemcpyAsync(stage_keys.as<unsigned>() + nfp, out_states.p, st.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		stage.reserve((size_t)nfp * (W + 1) * sizeof(unsigned));
+		MB_CUDA(cudaMemcpyAsync(stage.as<void>(), out_counts.p, nfp * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+		MB_CUDA(cudaMemcpyAsync(stage.as<unsigned>() + nfp, out_states.p, st.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
 		MB_CUDA(cudaStreamSynchronize(s));
-		std::copy_n(stage_keys.as<unsigned>(), nfp, cn.begin());
-		std::copy_n(stage_keys.as<unsigned>() + nfp, st.size(), st.begin());
+		std::copy_n(stage.as<unsigned>(), nfp, cn.begin());
+		std::copy_n(stage.as<unsigned>() + nfp, st.size(), st.begin());
 	}
 	else
 	{

@@ -93,29 +93,37 @@ struct dview
 	}
 };
 
-// Pinned host memory for the copies of a result. Allocating it takes 0.7 ms a MB, so a run's statistics keep
-// theirs, and it comes from and goes back to a pool of the process: blocks of power-of-two sizes, at most
-// 64 MB of them, the longest unused freed first. Any thread may borrow and return. Where pinning fails,
-// plain memory.
+// Pinned host memory for the copies of a result. Allocating it takes long (0.13 ms a MB from 2 MB on, 1 to 3 ms
+// for the first MB), so a run's statistics keep theirs, and it comes from and goes back to a pool of the
+// process: at most 64 MB, the longest unused freed first. Any thread may borrow and return. Where pinning
+// fails, plain memory.
 class host_stage
 {
 public:
+	struct block
+	{
+		void* p = nullptr;
+		size_t size = 0;
+		bool pinned = true;
+		void* base = nullptr; // of the mapping that p lies in (huge pages), and its bytes
+		size_t mapped = 0;
+	};
 	host_stage() = default;
 	~host_stage() { release(); }
 	host_stage(const host_stage&) = delete;
 	host_stage& operator=(const host_stage&) = delete;
 	void reserve(size_t bytes); // (what it held is lost)
+	void release() noexcept;	// gives the memory back
+	static void warm();			// 4 MB for the pool if it has none
+	size_t bytes() const { return b.size; }
 	template <typename T>
 	T* as(size_t offset = 0) const
 	{
-		return reinterpret_cast<T*>(static_cast<char*>(p) + offset);
+		return reinterpret_cast<T*>(static_cast<char*>(b.p) + offset);
 	}
 
 private:
-	void release() noexcept;
-	void* p = nullptr;
-	size_t size = 0;
-	bool pinned = true;
+	block b;
 };
 
 // Device scratch of sort_bins and compact_cells, kept between runs.
@@ -347,7 +355,10 @@ struct stats_state
 	dbuf bin_keys, bin_vals, out_bin_keys, out_bin_vals; // sparse bins (more than 20 non-internal nodes)
 	dbuf cell_idx, cell_vals; // non-zero cells of a large dense histogram (compact results), kept across runs
 	sort_scratch scratch;
-	host_stage stage, stage_keys, stage_vals; // a result's copies, kept across runs
+	// a result's copies, one after the other, kept across runs (the sorted sparse bins whatever their size; the cells of
+	// a compact histogram up to max_kept_stage bytes)
+	host_stage stage;
+	static constexpr size_t max_kept_stage = 1ull << 30;
 	unsigned bin_cap = 0;
 	bool wide = false;
 	bool has_tail = false; // occ is followed by the counts of mb_record_fixed (u32 per cell)

@@ -28,6 +28,7 @@ inline std::vector<copy> pending;
 inline std::map<void*, size_t> device, pinned; // live allocations
 inline std::function<void(const std::string& kernel, cudaStream_t, void** args, unsigned block, size_t smem)> on_launch;
 inline std::function<bool(size_t bytes)> fail_malloc; // true: this cudaMalloc fails
+inline bool fail_register = false;					  // host memory cannot be pinned
 inline std::string fail_function;					  // this kernel cannot be found
 inline cudaError_t last = cudaSuccess;
 
@@ -124,6 +125,18 @@ cudaError_t CUDARTAPI cudaHostAlloc(void** p, size_t n, unsigned)
 {
 	*p = std::malloc(n);
 	fake::pinned[*p] = n;
+	return cudaSuccess;
+}
+cudaError_t CUDARTAPI cudaHostRegister(void* p, size_t n, unsigned)
+{
+	if (fake::fail_register)
+		return fake::last = cudaErrorMemoryAllocation;
+	fake::pinned[p] = n;
+	return cudaSuccess;
+}
+cudaError_t CUDARTAPI cudaHostUnregister(void* p)
+{
+	fake::pinned.erase(p);
 	return cudaSuccess;
 }
 cudaError_t CUDARTAPI cudaFreeHost(void* p)

@@ -116,6 +116,46 @@ void family_loads_after_a_failure()
 	}
 }
 
+// Staging memory: hardly more than was asked for, reused for requests of about its size, at most 64 MB of it kept
+// when nobody holds any, and plain memory where pinning fails.
+void staging_memory_is_bounded()
+{
+	const size_t mb = 1 << 20;
+	for (size_t bytes : { (size_t)1, 5000 * (size_t)1, mb + 1, 3 * mb, 65 * mb, 130 * mb })
+	{
+		mb::host_stage s;
+		s.reserve(bytes);
+		CHECK(s.bytes() >= bytes && s.bytes() <= std::max(2 * mb, bytes) * 5 / 4 + 2 * mb);
+		std::memset(s.as<char>(), 1, bytes);
+		CHECK(reinterpret_cast<uintptr_t>(s.as<char>()) % 16 == 0);
+	}
+	CHECK(fake::held(fake::pinned) <= 64 * mb);
+	{
+		mb::host_stage a;
+		a.reserve(20 * mb);
+		const void* was = a.as<void>();
+		a.release();
+		mb::host_stage b;
+		b.reserve(21 * mb);
+		CHECK(b.as<void>() == was);
+		mb::host_stage c;
+		c.reserve(100000); // (not the large one)
+		CHECK(c.bytes() < 4 * mb);
+	}
+	{
+		std::vector<mb::host_stage> many(12);
+		for (mb::host_stage& x : many)
+			x.reserve(20 * mb);
+	}
+	CHECK(fake::held(fake::pinned) <= 64 * mb);
+	fake::fail_register = true;
+	mb::host_stage plain;
+	plain.reserve(500 * mb);
+	std::memset(plain.as<char>(), 1, 500 * mb);
+	CHECK(fake::held(fake::pinned) <= 64 * mb);
+	fake::fail_register = false;
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -123,6 +163,7 @@ int main(int argc, char** argv)
 	const std::map<std::string, void (*)()> checks = {
 		{ "jump_table_is_there_before_the_first_launch", jump_table_is_there_before_the_first_launch },
 		{ "family_loads_after_a_failure", family_loads_after_a_failure },
+		{ "staging_memory_is_bounded", staging_memory_is_bounded },
 	};
 	for (int i = 1; i < argc; i++)
 		checks.at(argv[i])();

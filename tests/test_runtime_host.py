@@ -1,5 +1,5 @@
-"""The host runtime without a GPU: order of uploads, loading after a failure, on the stand-in for CUDA of
-tests/cpp/fake_cuda.h."""
+"""The host runtime without a GPU: order of uploads, loading after a failure, bounds of what is kept, on the stand-in
+for CUDA of tests/cpp/fake_cuda.h."""
 import os
 import subprocess
 
@@ -20,7 +20,8 @@ def runtime_test(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["jump_table_is_there_before_the_first_launch", "family_loads_after_a_failure"])
+@pytest.mark.parametrize("check", ["jump_table_is_there_before_the_first_launch", "family_loads_after_a_failure",
+                                   "staging_memory_is_bounded"])
 def test_runtime(runtime_test, check):
     p = subprocess.run([runtime_test, check], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, p.stdout + p.stderr
