@@ -506,33 +506,41 @@ __device__ void mbb_body(const mb_batch_params& B)
 			}
 		}
 
+		// trajectories at a fixed point end: the state stays until max_time. All lanes meet again before the others'
+		// step: as a branch of the step, with its end, the compiler let the lanes that took it and the others run on
+		// apart (a 48-node network whose trajectories end so after 35 steps, 3e5 of them: 4.1 ms, 3.0 so)
+		if (running && total == 0)
+		{
+			const mb_variant& var = B.vars[vi];
+			const NET net(B, var);
+			const bool discrete = net.discrete();
+			const float max_time = net.max_time();
+			running = false;
+			mbb_record<GRAD>(var, var.st.win_h, v, P, acc, idx, time, max_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
+			atomicAdd(var.st.final_cnt + idx, 1u);
+			unsigned st[64];
+			const int W = net.W() < 64 ? net.W() : 64;
+			for (int w = 0; w < W; w++)
+				st[w] = v.S(w);
+			mb_fixed_insert_rt(var.st, st, W);
+			if (GRAD)
+				mbb_grad_end(v, P, discrete, C1, C2);
+			atomicAdd(var.transitions, trans + (max_time != 0.f ? 1 : 0)); // (steps that end at time 0 are empty)
+			trans = 0;
+		}
+		__syncwarp();
+
 		// steps per pass of the work-fetch loop: several (as in the fast kernel) only in the
 		// specialised gradient kernel (the gradient on the 50-node network 21.5 -> 20.6 ms); the
 		// specialised forward kernel lost 3.5 % with them, and the ahead-of-time kernels spilled 62
 		// bytes and halved the throughput of the 256-variant sweep
-		for (int step = 0; step < (GRAD ? NET::steps_per_pass() : 1) && running; step++)
+		constexpr int steps = GRAD ? NET::steps_per_pass() : 1;
+		for (int step = 0; step < steps && running && (step == 0 || total != 0); step++)
 		{
 			const mb_variant& var = B.vars[vi];
 			const NET net(B, var);
 			const bool discrete = net.discrete();
 			const float max_time = net.max_time(), tick = net.tick();
-			if (total == 0)
-			{
-				// a fixed point: the state stays until max_time
-				running = false;
-				mbb_record<GRAD>(var, var.st.win_h, v, P, acc, idx, time, max_time, 0.f, true, discrete, var.st.win_tick, C1, C2, cc);
-				atomicAdd(var.st.final_cnt + idx, 1u);
-				unsigned st[64];
-				const int W = net.W() < 64 ? net.W() : 64;
-				for (int w = 0; w < W; w++)
-					st[w] = v.S(w);
-				mb_fixed_insert_rt(var.st, st, W);
-				if (GRAD)
-					mbb_grad_end(v, P, discrete, C1, C2);
-				atomicAdd(var.transitions, trans + (max_time != 0.f ? 1 : 0)); // (steps that end at time 0 are empty)
-				trans = 0;
-				break;
-			}
 			const uint4 rb = curand4(&rng);
 			float tn;
 			if (discrete)

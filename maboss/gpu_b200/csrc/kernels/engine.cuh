@@ -1270,7 +1270,10 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_param
 		}
 
 		// up to MB_STEPS_PER_PASS steps of a running trajectory per pass of the work-fetch loop
-		// (+1.6 % on the 1000-node network; as in the fast kernel)
+		// (+1.6 % on the 1000-node network; as in the fast kernel). The ends are branches without a break: behind
+		// one the compiler lets the lanes that go on run apart (a 48-node network whose trajectories end at fixed
+		// points after 35 steps, 3e5 of them in fast mode: 4.1 ms with a break, 2.9 without; 1e5 in exact mode 1.46,
+		// 1.15)
 		for (int step = 0; step < MB_STEPS_PER_PASS && running; step++)
 		{
 			const float total = mb_exact_total(v, lo);
@@ -1281,9 +1284,8 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_param
 				atomicAdd(P.errors, 1u);
 				running = false;
 				mb_final_add(P.st, idx);
-				break;
 			}
-			if (total == 0.f)
+			else if (total == 0.f)
 			{
 				// a fixed point: the state stays until max_time
 				running = false;
@@ -1294,38 +1296,40 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 1) mb_fused_exact(mb_fused_param
 				for (int w = 0; w < state_words; w++)
 					st[w] = v.S(w);
 				mb_fixed_insert(P.st, st);
-				break;
-			}
-			float tn;
-			if (discrete_time)
-			{
-				tn = time + time_tick;
-				tn = max_time - time_tick < tn ? max_time : tn;
 			}
 			else
-				tn = time + -logf(curand_uniform(&rng)) / total;
-			tn = fminf(tn, max_time);
-			if (h_stale)
-				h_cache = mb_exact_entropy(v);
-			h_stale = false;
-			trans += (tn != 0.f) ? 1ull : 0ull;
-			if (tn != 0.f)
 			{
+				float tn;
 				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, h_cache);
+				{
+					tn = time + time_tick;
+					tn = max_time - time_tick < tn ? max_time : tn;
+				}
 				else
-					mb_record_cont(acc, P.st, hsink, idx, time, tn, h_cache);
+					tn = time + -logf(curand_uniform(&rng)) / total;
+				tn = fminf(tn, max_time);
+				if (h_stale)
+					h_cache = mb_exact_entropy(v);
+				h_stale = false;
+				trans += (tn != 0.f) ? 1ull : 0ull;
+				if (tn != 0.f)
+				{
+					if (discrete_time)
+						mb_record_disc(P.st, hsink, idx, time, h_cache);
+					else
+						mb_record_cont(acc, P.st, hsink, idx, time, tn, h_cache);
+				}
+				time = tn;
+				if (time >= max_time)
+				{
+					running = false;
+					mb_final_add(P.st, idx);
+				}
+				else if (P.traj_len > 1 && ++slot >= P.traj_len)
+					slot = 1; // epoch boundary: the next epoch re-evaluates the same state
+				else
+					lo = mb_exact_flip(v, mb_exact_select(v, curand_uniform(&rng) * total), idx, h_stale);
 			}
-			time = tn;
-			if (time >= max_time)
-			{
-				running = false;
-				mb_final_add(P.st, idx);
-			}
-			else if (P.traj_len > 1 && ++slot >= P.traj_len)
-				slot = 1; // epoch boundary: the next epoch re-evaluates the same state
-			else
-				lo = mb_exact_flip(v, mb_exact_select(v, curand_uniform(&rng) * total), idx, h_stale);
 		}
 		__syncwarp();
 	}
@@ -1663,155 +1667,157 @@ extern "C" __global__ void MB_FUSED_BOUNDS(128, 5) mb_fused_fast(mb_fused_params
 				for (int w = 0; w < state_words; w++)
 					st[w] = v.S(w);
 				mb_fixed_insert(P.st, st);
-				break;
-			}
-			const uint4 rb = curand4(&rng); // x: waiting time, (y, z): flip
-			float tn;
-			if (discrete_time)
-			{
-				tn = time + time_tick;
-				tn = max_time - time_tick < tn ? max_time : tn;
 			}
 			else
 			{
-				// uniform in (0, 1]: the top 24 bits plus one, times 2^-24
-				const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
-				tn = time + -logf(u) / ((float)total * inv_scale);
-			}
-			tn = fminf(tn, max_time);
-			trans += (tn != 0.f) ? 1ull : 0ull;
-			if (tn != 0.f)
-			{
+				const uint4 rb = curand4(&rng); // x: waiting time, (y, z): flip
+				float tn;
 				if (discrete_time)
-					mb_record_disc(P.st, hsink, idx, time, h);
+				{
+					tn = time + time_tick;
+					tn = max_time - time_tick < tn ? max_time : tn;
+				}
 				else
-					mb_record_cont(acc, P.st, hsink, idx, time, tn, h);
-			}
-			time = tn;
-			if (time >= max_time)
-			{
-				running = false;
-				mb_final_add(P.st, idx);
-			}
-			else
-			{
-				// draw the flip: r uniform in [0, total), then group -> word -> node
-				const unsigned long long r = __umul64hi(((unsigned long long)rb.y << 32) | rb.z, total);
-				// gs holds inclusive prefix sums over the groups: the flip's group is the number of
-				// prefixes <= r, counted with independent comparisons (a chain of additions before:
-				// +2.4 % on the 1000-node network, same selection)
-				unsigned long long cum = 0;
-				int g = 0;
-#pragma unroll
-				for (int i = 0; i < MB_GROUPS - 1; i++)
 				{
-					const bool le = gs[i] <= r;
-					g += le ? 1 : 0;
-					cum = le ? gs[i] : cum;
+					// uniform in (0, 1]: the top 24 bits plus one, times 2^-24
+					const float u = (float)((rb.x >> 8) + 1u) * 5.9604644775390625e-8f;
+					tn = time + -logf(u) / ((float)total * inv_scale);
 				}
-				// the group's word sums are loaded together (independent shared-memory loads), their
-				// prefix sums formed as a tree (3 levels for 8 words) and the chosen word counted with
-				// independent comparisons (+1.5 % on the 1000-node network over a compare-and-add chain,
-				// which was +2.3 % over a load-compare loop; same selection)
-				int word = g * MB_WPG;
+				tn = fminf(tn, max_time);
+				trans += (tn != 0.f) ? 1ull : 0ull;
+				if (tn != 0.f)
 				{
-					unsigned long long pq[MB_WPG];
+					if (discrete_time)
+						mb_record_disc(P.st, hsink, idx, time, h);
+					else
+						mb_record_cont(acc, P.st, hsink, idx, time, tn, h);
+				}
+				time = tn;
+				if (time >= max_time)
+				{
+					running = false;
+					mb_final_add(P.st, idx);
+				}
+				else
+				{
+					// draw the flip: r uniform in [0, total), then group -> word -> node
+					const unsigned long long r = __umul64hi(((unsigned long long)rb.y << 32) | rb.z, total);
+					// gs holds inclusive prefix sums over the groups: the flip's group is the number of
+					// prefixes <= r, counted with independent comparisons (a chain of additions before:
+					// +2.4 % on the 1000-node network, same selection)
+					unsigned long long cum = 0;
+					int g = 0;
 #pragma unroll
-					for (int i = 0; i < MB_WPG; i++)
+					for (int i = 0; i < MB_GROUPS - 1; i++)
 					{
-						const int w = g * MB_WPG + i;
-						pq[i] = w < state_words ? (unsigned long long)v.Q(w) : 0ull;
+						const bool le = gs[i] <= r;
+						g += le ? 1 : 0;
+						cum = le ? gs[i] : cum;
 					}
-#pragma unroll
-					for (int d = 1; d < MB_WPG; d <<= 1)
-#pragma unroll
-						for (int i = MB_WPG - 1; i >= d; i--)
-							pq[i] += pq[i - d];
-					const unsigned long long rr = r - cum;
-					int k = 0;
-					unsigned long long c = 0;
-#pragma unroll
-					for (int i = 0; i < MB_WPG - 1; i++)
+					// the group's word sums are loaded together (independent shared-memory loads), their
+					// prefix sums formed as a tree (3 levels for 8 words) and the chosen word counted with
+					// independent comparisons (+1.5 % on the 1000-node network over a compare-and-add chain,
+					// which was +2.3 % over a load-compare loop; same selection)
+					int word = g * MB_WPG;
 					{
-						const bool le = pq[i] <= rr && g * MB_WPG + i + 1 < state_words;
-						k += le ? 1 : 0;
-						c = le ? pq[i] : c;
+						unsigned long long pq[MB_WPG];
+#pragma unroll
+						for (int i = 0; i < MB_WPG; i++)
+						{
+							const int w = g * MB_WPG + i;
+							pq[i] = w < state_words ? (unsigned long long)v.Q(w) : 0ull;
+						}
+#pragma unroll
+						for (int d = 1; d < MB_WPG; d <<= 1)
+#pragma unroll
+							for (int i = MB_WPG - 1; i >= d; i--)
+								pq[i] += pq[i - d];
+						const unsigned long long rr = r - cum;
+						int k = 0;
+						unsigned long long c = 0;
+#pragma unroll
+						for (int i = 0; i < MB_WPG - 1; i++)
+						{
+							const bool le = pq[i] <= rr && g * MB_WPG + i + 1 < state_words;
+							k += le ? 1 : 0;
+							c = le ? pq[i] : c;
+						}
+						word = g * MB_WPG + k;
+						cum += c;
 					}
-					word = g * MB_WPG + k;
-					cum += c;
-				}
-				const uint32_t sw = v.S(word);
-				uint32_t um = v.U(word);
-				int j = 32 * word + 31 - __clz(um | 1u);
-				// the chosen word's unstable nodes two at a time: both rate loads are issued before
-				// the first comparison (+1.9 % on the 1000-node network over one load per step)
-				while (um)
-				{
-					const int b0 = __ffs(um) - 1;
-					const uint32_t um1 = um & (um - 1u);
-					const int b1 = um1 ? __ffs(um1) - 1 : b0;
-					const uint2 qq0 = mb_q(v, 32 * word + b0);
-					const uint2 qq1 = mb_q(v, 32 * word + b1);
-					const uint32_t qa = ((sw >> b0) & 1u) ? qq0.y : qq0.x;
-					j = 32 * word + b0;
-					if (r < cum + qa)
-						break;
-					cum += qa;
-					if (!um1)
-						break;
-					const uint32_t qb = ((sw >> b1) & 1u) ? qq1.y : qq1.x;
-					j = 32 * word + b1;
-					if (r < cum + qb)
-						break;
-					cum += qb;
-					um = um1 & (um1 - 1u);
-				}
-				const uint2 nj = mb_deps(v, j);
+					const uint32_t sw = v.S(word);
+					uint32_t um = v.U(word);
+					int j = 32 * word + 31 - __clz(um | 1u);
+					// the chosen word's unstable nodes two at a time: both rate loads are issued before
+					// the first comparison (+1.9 % on the 1000-node network over one load per step)
+					while (um)
+					{
+						const int b0 = __ffs(um) - 1;
+						const uint32_t um1 = um & (um - 1u);
+						const int b1 = um1 ? __ffs(um1) - 1 : b0;
+						const uint2 qq0 = mb_q(v, 32 * word + b0);
+						const uint2 qq1 = mb_q(v, 32 * word + b1);
+						const uint32_t qa = ((sw >> b0) & 1u) ? qq0.y : qq0.x;
+						j = 32 * word + b0;
+						if (r < cum + qa)
+							break;
+						cum += qa;
+						if (!um1)
+							break;
+						const uint32_t qb = ((sw >> b1) & 1u) ? qq1.y : qq1.x;
+						j = 32 * word + b1;
+						if (r < cum + qb)
+							break;
+						cum += qb;
+						um = um1 & (um1 - 1u);
+					}
+					const uint2 nj = mb_deps(v, j);
 
-				// flip j and re-evaluate it and the nodes whose logic reads it
-				v.S(j >> 5) ^= 1u << (j & 31);
-				const int pj = (int)(nj.y >> 16) - 1;
-				if (pj >= 0)
-					idx ^= (mb_idx_t)1 << pj;
-				bool ni_changed = pj >= 0;
-				const int d0 = (int)nj.x, d1 = d0 + (int)(nj.y & 0xffffu);
-				// the dependents of one flip are distinct nodes: their records are evaluated
-				// independently, two at a time so that both records' loads are in flight together
-				auto dependent = [&](int d, const uint4& rec) {
-					const int k = (int)(rec.x & 0xffffu);
-					const uint2 qk = mb_q(v, k);
-					const int wk = k >> 5;
-					const uint32_t bk = 1u << (k & 31);
-					const bool on = (v.S(wk) & bk) != 0;
-					const bool was_on = (k == j) ? !on : on;
-					const uint32_t uw = v.U(wk);
-					const bool was_unstable = (uw & bk) != 0;
-					const bool unstable = on != mb_incr_logic(v, d, rec);
-					const uint32_t qo = was_unstable ? (was_on ? qk.y : qk.x) : 0u;
-					const uint32_t qn = unstable ? (on ? qk.y : qk.x) : 0u;
-					if (unstable != was_unstable)
-						v.U(wk) = uw ^ bk;
-					if (qn != qo)
+					// flip j and re-evaluate it and the nodes whose logic reads it
+					v.S(j >> 5) ^= 1u << (j & 31);
+					const int pj = (int)(nj.y >> 16) - 1;
+					if (pj >= 0)
+						idx ^= (mb_idx_t)1 << pj;
+					bool ni_changed = pj >= 0;
+					const int d0 = (int)nj.x, d1 = d0 + (int)(nj.y & 0xffffu);
+					// the dependents of one flip are distinct nodes: their records are evaluated
+					// independently, two at a time so that both records' loads are in flight together
+					auto dependent = [&](int d, const uint4& rec) {
+						const int k = (int)(rec.x & 0xffffu);
+						const uint2 qk = mb_q(v, k);
+						const int wk = k >> 5;
+						const uint32_t bk = 1u << (k & 31);
+						const bool on = (v.S(wk) & bk) != 0;
+						const bool was_on = (k == j) ? !on : on;
+						const uint32_t uw = v.U(wk);
+						const bool was_unstable = (uw & bk) != 0;
+						const bool unstable = on != mb_incr_logic(v, d, rec);
+						const uint32_t qo = was_unstable ? (was_on ? qk.y : qk.x) : 0u;
+						const uint32_t qn = unstable ? (on ? qk.y : qk.x) : 0u;
+						if (unstable != was_unstable)
+							v.U(wk) = uw ^ bk;
+						if (qn != qo)
+						{
+							const long long dq = (long long)qn - (long long)qo;
+							v.Q(wk) += (uint32_t)dq;
+							mb_group_add(gs, wk / MB_WPG, dq);
+							total += (unsigned long long)dq;
+						}
+						if (qn != qo || unstable != was_unstable)
+							ni_changed |= ((rec.x >> 21) & 127u) != 0u;
+					};
+					for (int d = d0; d < d1; d += 2)
 					{
-						const long long dq = (long long)qn - (long long)qo;
-						v.Q(wk) += (uint32_t)dq;
-						mb_group_add(gs, wk / MB_WPG, dq);
-						total += (unsigned long long)dq;
+						const bool two = d + 1 < d1;
+						const uint4 rec0 = mb_rec(v, d);
+						const uint4 rec1 = two ? mb_rec(v, d + 1) : make_uint4(0u, 0u, 0u, 0u);
+						dependent(d, rec0);
+						if (two)
+							dependent(d + 1, rec1);
 					}
-					if (qn != qo || unstable != was_unstable)
-						ni_changed |= ((rec.x >> 21) & 127u) != 0u;
-				};
-				for (int d = d0; d < d1; d += 2)
-				{
-					const bool two = d + 1 < d1;
-					const uint4 rec0 = mb_rec(v, d);
-					const uint4 rec1 = two ? mb_rec(v, d + 1) : make_uint4(0u, 0u, 0u, 0u);
-					dependent(d, rec0);
-					if (two)
-						dependent(d + 1, rec1);
+					if (ni_changed)
+						h = mb_incr_entropy(v);
 				}
-				if (ni_changed)
-					h = mb_incr_entropy(v);
 			}
 		}
 		__syncwarp();
