@@ -212,9 +212,11 @@ __device__ __forceinline__ void mb_fused_body(const mb_fused_params& P)
 	unsigned long long trans = 0;
 	mb_win_acc acc;
 	mb_acc_init(acc);
-	for (; (int)(threadIdx.x & 31) < P.lanes;)
+	// (lanes without trajectories find the work exhausted: as a condition of the loop, or in front of it, their number
+	// took some networks' kernels from 128 registers to 150 and more, so from two blocks an SM to one)
+	for (;;)
 	{
-		const unsigned long long t = atomicAdd(P.next_traj, 1ull);
+		const unsigned long long t = (int)(threadIdx.x & 31) < P.lanes ? atomicAdd(P.next_traj, 1ull) : ~0ull;
 		if (t >= P.n_traj)
 			break;
 		const unsigned long long id = P.first_traj + t;

@@ -1195,7 +1195,17 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 					   !st.wide && (size_t)st.n_windows * st.n_bins <= 4096;
 	if (P.st.cnt_in_smem)
 		smem += (size_t)st.n_windows * st.n_bins * sizeof(unsigned);
-	if (c.mode == MB_MODE_FUSED_EXACT ? m.incremental : m.fast_incremental())
+	const bool dense = !(c.mode == MB_MODE_FUSED_EXACT ? m.incremental : m.fast_incremental());
+	if (dense && block == 256 && c.blocks_per_sm <= 0)
+	{
+		// (no smaller shape asked for) a kernel of more than 128 registers has one block of 256 threads on an SM: smaller
+		// ones leave fewer registers unused
+		int most = occupancy_blocks(f, 256, smem) * 256;
+		for (int b : { 192, 128 })
+			if (most < 512 && occupancy_blocks(f, b, smem) * b > most)
+				most = occupancy_blocks(f, b, smem) * b, block = b;
+	}
+	if (!dense)
 	{
 		// per thread in shared memory: state words, unstable masks and word rate sums; or per warp its array
 		constexpr size_t max_smem = 227 * 1024;
@@ -1222,7 +1232,7 @@ unsigned launch_fused(module& m, const run_config& c, stats_state& st, long long
 	cu_throw(drv().FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_PREFERRED_SHARED_MEMORY_CARVEOUT, carve),
 			 "cuFuncSetAttribute");
 	const int per_sm = c.blocks_per_sm > 0 ? c.blocks_per_sm : occupancy_blocks(f, block, smem);
-	P.lanes = lanes_per_warp(n, m.ctx->sm_count);
+	P.lanes = dense && m.state_words > max_spread_words ? 32 : lanes_per_warp(n, m.ctx->sm_count);
 	const long long per_block = (long long)(block / 32) * P.lanes, needed = (n + per_block - 1) / per_block;
 	const unsigned grid = (unsigned)std::max(1LL, std::min<long long>(needed, (long long)per_sm * m.ctx->sm_count));
 	void* args[] = { &P };

@@ -42,6 +42,11 @@ inline int lanes_per_warp(long long n, int sm_count)
 	return lanes < 1 ? 1 : lanes > 32 ? 32 : (int)lanes;
 }
 
+// The dense kernels of larger networks are not spread: a step is the code of every node, more than an SM's instruction
+// caches hold, which all SMs then fetch at once. Fast mode, 1e3 trajectories, in full warps -> spread, ms: 120 nodes
+// 0.87 -> 0.55, 200 nodes 3.0 -> 2.5, 400 nodes 41 -> 48 and (another network) 19 -> 40.
+constexpr int max_spread_words = 8;
+
 // mb_initialize_random: consecutive trajectories per warp and the grid for n trajectories. One per warp until
 // the chip has 32 warps an SM to hide the latency of the jumps to each warp's first trajectory, then as
 // many as keep that number of warps, up to 128 (the jumps are then a twentieth of the work).
