@@ -1101,7 +1101,14 @@ std::string generate_code(const model_t& m)
 	ss << "    return h > 0.f ? h : 0.f;" << std::endl << "}" << std::endl;
 
 	emit_incremental_tables(ss, L);
-	if (!emit_gates(ss, m, L) && L.incremental_ok)
+	const bool gates = emit_gates(ss, m, L);
+	// Epoch mode of models whose logics of 13 to 16 inputs are no gates: the dense kernel in small networks. An epoch of
+	// 1e3 trajectories, and of 3e4, incremental | dense, ms: 40 nodes 0.87 | 0.50, 1.08 | 0.63, 80 nodes 1.19 | 0.77,
+	// 1.42 | 0.91, 128 nodes 1.93 | 1.69, 2.25 | 1.89, 200 nodes 2.96 | 3.41, 3.58 | 3.89
+	constexpr int dense_epoch_words = 5;
+	if (!gates && L.incremental_ok && L.max_inputs > incremental_record_inputs && L.state_words <= dense_epoch_words)
+		ss << "#define MBG_EPOCH_DENSE 1" << std::endl;
+	if (!gates && L.incremental_ok)
 	{
 		// the fused kernels' tables in shared memory, if at least 256 threads' rows fit beside them and the
 		// entropy sums (640 threads at most: 102 registers each)

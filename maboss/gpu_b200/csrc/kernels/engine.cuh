@@ -14,9 +14,13 @@
 // every sum independent of thread order, so results are reproducible bit for bit.
 #include <curand_kernel.h>
 
-// logics of 13 to 16 inputs: incremental exact and epoch kernels, dense fast kernel
+// logics of 13 to 16 inputs: incremental exact and epoch kernels (the latter not where generated MBG_EPOCH_DENSE),
+// dense fast kernel
 #ifdef MBG_INCREMENTAL_MANY
 #define MBG_INCREMENTAL 1
+#endif
+#if defined(MBG_EPOCH_DENSE) && !defined(MB_EPOCH_DENSE)
+#define MB_EPOCH_DENSE 1
 #endif
 
 enum class trajectory_status : uint8_t

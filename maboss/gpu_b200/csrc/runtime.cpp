@@ -494,6 +494,7 @@ std::unique_ptr<module> compile_module(context& ctx, const std::string& generate
 	m->incremental = generated_code.find("#define MBG_INCREMENTAL 1") != std::string::npos ||
 					 generated_code.find("#define MBG_INCREMENTAL_MANY 1") != std::string::npos;
 	m->integer_rates = generated_code.find("#define MBG_INTEGER_RATES 1") != std::string::npos;
+	m->dense_epochs = generated_code.find("#define MBG_EPOCH_DENSE 1") != std::string::npos;
 	m->gate_words = parse_constexpr(generated_code, "mbg_gate_words", 0);
 	m->table_threads = parse_constexpr(generated_code, "mbg_table_threads", 0);
 	m->table_bytes = (size_t)parse_constexpr(generated_code, "mbg_table_bytes", 0);
@@ -1258,7 +1259,7 @@ void simulate_epoch(module& m, bool dense, cudaStream_t s, int n, int stride, in
 		return;
 	}
 	m.ensure(FAMILY_EPOCH);
-	if (!m.incremental)
+	if (!m.incremental || m.dense_epochs)
 	{
 		launch(m.sim_epoch, (n + 255) / 256, 256, 0, s, a);
 		return;

@@ -189,6 +189,7 @@ struct module
 	int noninternal_count = -1; // from the generated code (mbg_noninternal_count), -1 if absent
 	bool incremental = false;	// @logic-form model: exact and epoch modes use the incremental kernels (generated MBG_INCREMENTAL)
 	bool integer_rates = false; // fast mode's incremental kernel too (generated MBG_INTEGER_RATES), else its dense kernel
+	bool dense_epochs = false; // epoch mode's dense kernel all the same (generated MBG_EPOCH_DENSE)
 	bool fast_incremental() const { return incremental && integer_rates; }
 	// words of a warp's array in the lockstep kernels (generated MBG_GATES), 0: the incremental kernels
 	int gate_words = 0;
