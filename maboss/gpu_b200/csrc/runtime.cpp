@@ -384,8 +384,89 @@ void dbuf::alloc(size_t n)
 	bytes = 0;
 	if (n == 0)
 		return;
-	MB_CUDA(cudaMalloc(&p, n));
+	cudaError_t e = cudaMalloc(&p, n);
+	if (e == cudaErrorMemoryAllocation && kept_buffers::give_back())
+	{
+		(void)cudaGetLastError();
+		e = cudaMalloc(&p, n);
+	}
+	if (e != cudaSuccess)
+		p = nullptr;
+	cuda_throw(e, "cudaMalloc");
 	bytes = n;
+}
+
+namespace {
+// the kept buffers of the process, the longest unused first (never destroyed: objects may outlive it)
+struct kept_list
+{
+	std::mutex mu;
+	std::vector<kept_buffers*> all;
+};
+kept_list& kept()
+{
+	static kept_list* list = new kept_list;
+	return *list;
+}
+} // namespace
+
+kept_buffers::kept_buffers()
+{
+	std::lock_guard<std::mutex> lk(kept().mu);
+	kept().all.push_back(this);
+}
+
+void kept_buffers::forget()
+{
+	std::lock_guard<std::mutex> lk(kept().mu);
+	std::vector<kept_buffers*>& all = kept().all;
+	all.erase(std::find(all.begin(), all.end(), this));
+}
+
+// (with the list's mutex held, and the device current)
+bool kept_buffers::trim(int device, size_t most)
+{
+	size_t total = 0;
+	bool freed = false;
+	for (const kept_buffers* b : kept().all)
+		total += b->device == device && b->users == 0 ? b->held() : 0;
+	for (kept_buffers* b : kept().all)
+		if (total > most && b->device == device && b->users == 0 && b->held() > 0)
+		{
+			total -= b->held();
+			b->drop();
+			freed = true;
+		}
+	return freed;
+}
+
+bool kept_buffers::give_back()
+{
+	int device = 0;
+	if (cudaGetDevice(&device) != cudaSuccess)
+		return false;
+	std::lock_guard<std::mutex> lk(kept().mu);
+	return trim(device, 0);
+}
+
+kept_use::kept_use(kept_buffers& buffers, int device, size_t most_bytes) : b(buffers), most(most_bytes)
+{
+	std::lock_guard<std::mutex> lk(kept().mu);
+	b.device = device;
+	b.users++;
+	std::vector<kept_buffers*>& all = kept().all;
+	const auto it = std::find(all.begin(), all.end(), &b);
+	std::rotate(it, it + 1, all.end());
+}
+
+kept_use::~kept_use()
+{
+	std::lock_guard<std::mutex> lk(kept().mu);
+	if (--b.users > 0)
+		return;
+	if (b.held() > most)
+		b.drop();
+	kept_buffers::trim(b.device, kept_buffers::max_idle);
 }
 
 context::context(int dev) : device(dev)
@@ -863,6 +944,7 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 	r.fx_h = fx_h;
 	r.sections = sections;
 	r.wide = wide;
+	kept_use use(scratch, m.ctx->device, sort_scratch::most);
 	const size_t cells = (size_t)n_windows * n_bins;
 	// compact the occupied fixed-point slots on the device; the same launch adds the window sums of the
 	// trajectories that were counted at their fixed point (and clears the counts)
@@ -925,7 +1007,6 @@ std::unique_ptr<result> stats_state::finalize(long long n, cudaStream_t s)
 		}
 		decode_sorted_bins(stage.as<uint64_t>(), stage.as<long long>(at_vals), nb, n_windows, (int)std::thread::hardware_concurrency(),
 						   r.sp_w, r.sp_idx, r.sp_val, r.sp_begin, r.fin_idx, r.fin_cnt);
-		scratch.trim();
 		r.bin_overflow = ovf;
 	}
 	// a large dense histogram: only its non-zero cells (selected on the device in cell order), when
@@ -1323,7 +1404,7 @@ void run_epochs(module& m, const run_config& c, stats_state& st, epoch_buffers& 
 	const int B = (int)Bll;
 	if (E.batch != B) // (a runner's L and W do not change)
 	{
-		E = epoch_buffers();
+		E.drop();
 		for (int k = 0; k < 2; k++)
 		{
 			E.states[k].alloc((size_t)W * B * 4);
@@ -1336,7 +1417,6 @@ void run_epochs(module& m, const run_config& c, stats_state& st, epoch_buffers& 
 		E.statuses.alloc((size_t)B);
 		E.scratch.alloc(256 + partition_scratch_bytes(B));
 		E.batch = B;
-		E.bytes = (size_t)L * (W + 2) * B * 4;
 	}
 	dbuf &st0 = E.states[0], &st1 = E.states[1], &t0 = E.times[0], &t1 = E.times[1], &r0 = E.rands[0], &r1 = E.rands[1];
 	dbuf &ts = E.traj_states, &tt = E.traj_times, &th = E.traj_h, &stat = E.statuses, &scratch = E.scratch;
@@ -1432,9 +1512,22 @@ runner::runner(module& m, const run_config& c) : mod(&m), cfg(c)
 		rng_chunk = std::min(c.sample_count, max_rng_states);
 		if (m.incremental)
 			rng_chunk = std::max(1LL, std::min(rng_chunk, max_init_bytes / (4 * m.state_words)));
-		rng.alloc((size_t)rng_chunk * sizeof(curandState));
-		if (m.incremental)
-			init_states.alloc((size_t)4 * m.state_words * rng_chunk);
+		for (bool done = false; !done;)
+			try
+			{
+				rng.alloc((size_t)rng_chunk * sizeof(curandState));
+				if (m.incremental)
+					init_states.alloc((size_t)4 * m.state_words * rng_chunk);
+				done = true;
+			}
+			catch (const engine_error& e)
+			{
+				// less memory, more launches
+				if (e.code != MB_ERR_LIMIT || rng_chunk <= 1 << 16)
+					throw;
+				rng.alloc(0);
+				rng_chunk = (rng_chunk + 1) / 2;
+			}
 	}
 	MB_CUDA(cudaEventCreate(&ev0));
 	MB_CUDA(cudaEventCreate(&ev1));
@@ -1461,9 +1554,8 @@ void runner::launch(cudaStream_t s)
 	launches = 0;
 	if (cfg.mode == MB_MODE_EPOCH || cfg.mode == MB_MODE_EPOCH_DENSE)
 	{
+		kept_use use(epoch, mod->ctx->device, epoch_buffers::most); // (the last epoch is waited for)
 		run_epochs(*mod, cfg, st, epoch, cfg.sample_count, s, epochs, launches);
-		if (epoch.bytes > max_epoch_bytes)
-			epoch = epoch_buffers(); // (the last epoch has been waited for)
 	}
 	else
 	{

@@ -131,23 +131,68 @@ private:
 	block b;
 };
 
+// Device buffers that an object keeps between its calls only to spare the next call their allocation. While a call
+// uses them (kept_use) they are its own. The others are given back, by any thread, when an allocation on their
+// device fails; and together they hold at most max_idle bytes of a device, the longest unused going first.
+class kept_buffers
+{
+public:
+	kept_buffers();
+	kept_buffers(const kept_buffers&) = delete;
+	kept_buffers& operator=(const kept_buffers&) = delete;
+	virtual ~kept_buffers() = default;
+	virtual size_t held() const = 0;
+	virtual void drop() = 0;
+	// frees what is not in use on the current device; false: nothing was there
+	static bool give_back();
+	static constexpr size_t max_idle = 4ull << 30;
+
+protected:
+	void forget(); // (the first thing a destructor does)
+
+private:
+	friend class kept_use;
+	static bool trim(int device, size_t most);
+	int device = 0, users = 0;
+};
+
+// The scope of a call that uses kept buffers (whose work on the device has been waited for at its end). Above `most`
+// bytes they are freed at its end.
+class kept_use
+{
+public:
+	kept_use(kept_buffers& b, int device, size_t most);
+	~kept_use();
+	kept_use(const kept_use&) = delete;
+	kept_use& operator=(const kept_use&) = delete;
+
+private:
+	kept_buffers& b;
+	size_t most;
+};
+
 // Device scratch of sort_bins and compact_cells, kept between runs.
-struct sort_scratch
+struct sort_scratch : kept_buffers
 {
 	dbuf lo, lo_sorted, hi, hi_sorted, pos, pos_a, pos_b, tmp, counters, out_keys, out_vals;
+	static constexpr size_t most = 1ull << 30;
+	~sort_scratch() override { forget(); }
 	static void reserve(dbuf& b, size_t bytes)
 	{
 		if (b.bytes < bytes)
 			b.alloc(bytes + bytes / 4);
 	}
-	// gives back more than 1 GB (its work has been waited for)
-	void trim()
+	size_t held() const override
 	{
 		size_t total = 0;
-		for (const dbuf* b : { &lo, &lo_sorted, &hi, &hi_sorted, &pos, &pos_a, &pos_b, &tmp, &out_keys, &out_vals })
+		for (const dbuf* b : { &lo, &lo_sorted, &hi, &hi_sorted, &pos, &pos_a, &pos_b, &tmp, &counters, &out_keys, &out_vals })
 			total += b->bytes;
-		if (total > (1ull << 30))
-			*this = sort_scratch();
+		return total;
+	}
+	void drop() override
+	{
+		for (dbuf* b : { &lo, &lo_sorted, &hi, &hi_sorted, &pos, &pos_a, &pos_b, &tmp, &counters, &out_keys, &out_vals })
+			b->alloc(0);
 	}
 };
 
@@ -403,12 +448,31 @@ struct stats_state
 	std::unique_ptr<result> finalize(long long n_traj, cudaStream_t s);
 };
 
-// Device buffers of the epoch modes' batch (states, times, random states twice, trajectory slots).
-struct epoch_buffers
+// Device buffers of the epoch modes' batch (states, times, random states twice, trajectory slots). Kept for the next
+// launch where they take at most 4 GB: allocating and freeing the 0.2 GB of 1e5 trajectories of the 87-node
+// example model took 9 to 20 ms a run.
+struct epoch_buffers : kept_buffers
 {
 	dbuf states[2], times[2], rands[2], traj_states, traj_times, traj_h, statuses, scratch;
 	int batch = 0;
-	size_t bytes = 0;
+	static constexpr size_t most = 4ull << 30;
+	~epoch_buffers() override { forget(); }
+	size_t held() const override
+	{
+		size_t total = traj_states.bytes + traj_times.bytes + traj_h.bytes + statuses.bytes + scratch.bytes;
+		for (int k = 0; k < 2; k++)
+			total += states[k].bytes + times[k].bytes + rands[k].bytes;
+		return total;
+	}
+	void drop() override
+	{
+		batch = 0;
+		for (dbuf* b : { states, times, rands })
+			for (int k = 0; k < 2; k++)
+				b[k].alloc(0);
+		for (dbuf* b : { &traj_states, &traj_times, &traj_h, &statuses, &scratch })
+			b->alloc(0);
+	}
 };
 
 // A run whose device buffers are allocated once: launch() zeroes the accumulators and enqueues the
@@ -428,10 +492,7 @@ struct runner
 	long long rng_chunk = 0; // trajectories of a launch
 	static constexpr long long max_rng_states = 1LL << 24;
 	static constexpr long long max_init_bytes = 1LL << 30;
-	// epoch modes: kept for the next launch where they take at most 4 GB (allocating and freeing the 0.2 GB of
-	// 1e5 trajectories of the 87-node example model took 9 to 20 ms a run), else given back after each run
 	epoch_buffers epoch;
-	static constexpr size_t max_epoch_bytes = 4ull << 30;
 	runner(module& m, const run_config& c);
 	~runner();
 	void launch(cudaStream_t s);

@@ -156,6 +156,65 @@ void staging_memory_is_bounded()
 	fake::fail_register = false;
 }
 
+// Buffers kept between the runs of several modules: at most 4 GB in all, given back when another allocation fails,
+// and not while a run uses them.
+void kept_buffers_are_given_back()
+{
+	program a, b, c;
+	std::vector<std::unique_ptr<mb::runner>> runners;
+	const mb::run_config batch = a.config(MB_MODE_EPOCH, 1000000); // 1.3 GB of buffers
+	for (program* p : { &a, &b, &c })
+		for (int k = 0; k < 2; k++)
+		{
+			runners.push_back(std::make_unique<mb::runner>(*p->m, batch));
+			runners.back()->launch(p->ctx.stream);
+		}
+	size_t kept = 0;
+	for (const auto& r : runners)
+		kept += r->epoch.held();
+	CHECK(kept > 2500u << 20);
+	CHECK(kept <= mb::kept_buffers::max_idle);
+	CHECK(runners.back()->epoch.held() > 0 && runners.front()->epoch.held() == 0); // (the longest unused went first)
+
+	// a device that is full but for 100 MB: the next run's buffers come from those that wait
+	const size_t limit = fake::held(fake::device) + (100 << 20);
+	fake::fail_malloc = [&](size_t n) { return fake::held(fake::device) + n > limit; };
+	mb::runner more(*a.m, batch);
+	more.launch(a.ctx.stream);
+	CHECK(more.epoch.held() > 1u << 30);
+	CHECK(fake::held(fake::device) <= limit);
+	// no room at all: the run that fails does not take its own buffers away from under itself, and leaves none
+	const size_t full = fake::held(fake::device);
+	fake::fail_malloc = [&](size_t n) { return n > 1 << 20 && fake::held(fake::device) + n > full / 8; };
+	CHECK(throws([&] { runners[0]->launch(a.ctx.stream); }));
+	fake::fail_malloc = nullptr;
+	runners[0]->launch(a.ctx.stream);
+	CHECK(runners[0]->epoch.held() > 1u << 30);
+}
+
+// Exact runs whose random and initial states do not fit take more launches, which cover every trajectory once.
+void exact_run_in_more_launches_where_memory_is_short()
+{
+	program p;
+	long long next = 0, launches = 0;
+	fake::on_launch = [&](const std::string& kernel, cudaStream_t, void** args, unsigned, size_t) {
+		if (kernel != "mb_initialize_random")
+			return;
+		CHECK(*static_cast<unsigned long long*>(args[2]) == (unsigned long long)next);
+		next += *static_cast<int*>(args[0]);
+		launches++;
+	};
+	p.m->ensure(mb::FAMILY_EXACT);
+	fake::fail_malloc = [&](size_t n) { return n > 20u << 20; };
+	mb::run_config c = p.config(MB_MODE_FUSED_EXACT, 1000001);
+	c.fixed_capacity_log2 = 10;
+	mb::runner r(*p.m, c);
+	r.launch(p.ctx.stream);
+	CHECK(next == 1000001 && launches > 1);
+	fake::fail_malloc = nullptr;
+	fake::on_launch = nullptr;
+}
+
 } // namespace
 
 int main(int argc, char** argv)
@@ -164,6 +223,8 @@ int main(int argc, char** argv)
 		{ "jump_table_is_there_before_the_first_launch", jump_table_is_there_before_the_first_launch },
 		{ "family_loads_after_a_failure", family_loads_after_a_failure },
 		{ "staging_memory_is_bounded", staging_memory_is_bounded },
+		{ "kept_buffers_are_given_back", kept_buffers_are_given_back },
+		{ "exact_run_in_more_launches_where_memory_is_short", exact_run_in_more_launches_where_memory_is_short },
 	};
 	for (int i = 1; i < argc; i++)
 		checks.at(argv[i])();

@@ -21,7 +21,8 @@ def runtime_test(tmp_path_factory):
 
 
 @pytest.mark.parametrize("check", ["jump_table_is_there_before_the_first_launch", "family_loads_after_a_failure",
-                                   "staging_memory_is_bounded"])
+                                   "staging_memory_is_bounded", "kept_buffers_are_given_back",
+                                   "exact_run_in_more_launches_where_memory_is_short"])
 def test_runtime(runtime_test, check):
     p = subprocess.run([runtime_test, check], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, p.stdout + p.stderr
