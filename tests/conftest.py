@@ -17,6 +17,20 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a B200 (sm_100) GPU")
 
 
+# tests that read the reference build's numbers (the others of them say so themselves)
+NEED_REFERENCE_BUILD = {"test_reference_arm_prints_the_contract_line"}
+
+
+def pytest_collection_modifyitems(items):
+    from oracle import reference
+
+    if reference.available():
+        return
+    for item in items:
+        if item.name in NEED_REFERENCE_BUILD:
+            item.add_marker(pytest.mark.skip(reason="reference build absent (oracle/_ref)"))
+
+
 def model_files(name: str) -> tuple[str, str]:
     return os.path.join(MODELS, f"{name}.bnd"), os.path.join(MODELS, f"{name}.cfg")
 
