@@ -237,7 +237,11 @@ typedef struct mb_run_config_s
     unsigned long long first_traj; /* random-stream id of trajectory 0 (sharding / replicas) */
     int traj_len;                  /* epoch length (reference: trajectory_len_limit = 100) */
     int batch_limit;               /* epoch batch (reference: trajectory_batch_limit = 1e6) */
-    int block;                     /* threads per block (multiple of 32, <= 256) */
+    int block;                     /* threads per block (multiple of 32, <= 256). The kernels of rates in the @logic
+                                    * form take at most 128. With blocks_per_sm = 0 a value above 128 leaves the
+                                    * shape to the kernel: up to 640 threads in one block an SM where the network's
+                                    * tables are in shared memory; and 256 may become 192 or 128 in the kernels that
+                                    * evaluate every rate function, where more threads fit so */
     int blocks_per_sm;             /* 0 = occupancy calculator */
     int fixed_capacity_log2;       /* fixed-point table capacity, 0 = automatic */
     long long stats_trajectories;  /* 0, or the trajectory count of the whole job when this run is one

@@ -1111,7 +1111,10 @@ std::string generate_code(const model_t& m)
 	if (!gates && L.incremental_ok)
 	{
 		// the fused kernels' tables in shared memory, if at least 256 threads' rows fit beside them and the
-		// entropy sums (640 threads at most: 102 registers each)
+		// entropy sums (640 threads at most: 102 registers each). Against tables in global memory, fast mode 1e5 |
+		// exact 3e4 trajectories: 260 nodes 1.1x | 1.2, 400 nodes 1.04 to 1.2 | 1.15 to 1.2, 520 nodes 1.04 to 1.1 |
+		// 1.15 to 1.6, 700 nodes 1.0 | 1.5, 1000 nodes 1.0 (8 inputs a node) to 1.4 | 1.06 to 1.5; at most 256
+		// nodes whose logics are no gates 1.0 to 1.3 | 1.1 to 1.4
 		const size_t smem = 227 * 1024, tables = table_bytes(L);
 		const size_t h = (size_t)L.windows() * 8 <= 48 * 1024 ? (size_t)L.windows() * 8 : 0;
 		const size_t threads = tables + h < smem ? (smem - tables - h) / ((size_t)12 * L.state_words) / 32 * 32 : 0;

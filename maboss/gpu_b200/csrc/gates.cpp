@@ -498,8 +498,6 @@ gate_network build_gates(const model_t& m)
 	for (const gate& g : finals)
 		net.gates.push_back(resolved(g));
 	net.words = base + 32 * std::max(1, net.rounds);
-	// instructions of a step of 32 trajectories, about: 22 a round of gates, 20 a transposed word. Above,
-	// re-evaluating the flipped node's dependents alone is cheaper
 	net.ok = net.words < 8192 && 22 * (net.rounds + W) + 20 * W <= gate_max_cost;
 	return net;
 }

@@ -283,8 +283,6 @@ void simulate_epoch(module& m, bool dense, cudaStream_t s, int n, int stride, in
 					float* last_times, void* rands, unsigned* traj_states, float* traj_times, float* traj_h,
 					unsigned char* statuses, unsigned long long* transitions);
 
-// Sorts n sparse-bin records by their 128-bit keys (window, then non-internal index) on the device
-// (sort.cu); synchronises the stream.
 // The non-zero cells of a dense window histogram (`occ` int64 or `cnt` u32, whichever is not null), in
 // increasing cell order (window, then state): their cell indices into idx_out (u64) and values into
 // val_out (int64), both grown as needed. Returns the number of cells, or -1 without writing them
@@ -293,7 +291,8 @@ long long compact_cells(const long long* occ, const unsigned* cnt, unsigned long
 						unsigned long long max_entries, dbuf& idx_out, dbuf& val_out, int sm_count,
 						sort_scratch& scratch, cudaStream_t s);
 
-// (asynchronous; the sorted bins are in scratch.out_keys and scratch.out_vals)
+// Sorts n sparse-bin records by their 128-bit keys (window, then non-internal index) on the device (sort.cu).
+// Asynchronous; the sorted bins are in scratch.out_keys and scratch.out_vals.
 void sort_bins(const mb_key128* keys, const long long* vals, unsigned n, sort_scratch& scratch, cudaStream_t s);
 
 // Stable partition of the CONTINUE trajectories of an epoch batch into another buffer set
