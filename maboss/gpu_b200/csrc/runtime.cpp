@@ -325,14 +325,11 @@ void host_stage::reserve(size_t bytes)
 
 void host_stage::warm()
 {
-	stage_pool& pool = stages();
-	{
-		std::lock_guard<std::mutex> lk(pool.mu);
-		if (!pool.blocks.empty())
-			return;
-	}
-	host_stage s;
-	s.reserve(2 * huge_page - 2 * huge_page / 8);
+	static std::once_flag once;
+	std::call_once(once, [] {
+		host_stage s;
+		s.reserve(2 * huge_page - 2 * huge_page / 8);
+	});
 }
 
 void host_stage::release() noexcept
@@ -486,7 +483,7 @@ context::context(int dev) : device(dev)
 		throw engine_error(MB_ERR_NO_DEVICE, std::string("this engine is built for sm_100a (B200); device is ") +
 												 prop.name + " sm_" + std::to_string(cc_major) + std::to_string(cc_minor));
 	MB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-	host_stage::warm(); // 1 ms here, where making the context takes 900, so that small runs' first calls have it
+	host_stage::warm(); // 1 ms here, where making the first context takes 700 and more, for the first calls
 }
 
 context::~context()

@@ -119,7 +119,7 @@ public:
 	host_stage& operator=(const host_stage&) = delete;
 	void reserve(size_t bytes); // (what it held is lost)
 	void release() noexcept;	// gives the memory back
-	static void warm();			// 4 MB for the pool if it has none
+	static void warm();			// 4 MB for the pool, once in the process
 	size_t bytes() const { return b.size; }
 	template <typename T>
 	T* as(size_t offset = 0) const
