@@ -530,8 +530,10 @@ constexpr int MB_LW = state_words;
 constexpr bool MB_LOCK_SMALL = state_size <= 36;
 // Fast mode: a warp waits for this many lanes to start together while others run. Many where trajectories are
 // short and starting together is cheap, few where the passes that idle lanes wait through are long (gates).
-// 2 / 4 / 8 lanes, ms: 10 nodes 1e6 0.85 / 0.79 / 0.75, 50 nodes 1e6 5.54 / 5.49 / 5.63, 100 nodes 2e5 3.14 /
-// 3.11 / 3.15, the 87-node example model (8 rounds of gates) 2e5 4.64 / 4.69 / 4.70.
+// 2 / 4 / 8 lanes, ms: 10 nodes 1e6 0.85 / 0.79 / 0.74, 50 nodes 1e6 5.54 / 5.49 / 5.63, 100 nodes 2e5 3.14 /
+// 3.11 / 3.15, the 87-node example model (8 rounds of gates) 2e5 4.64 / 4.69 / 4.70; trajectories of unequal
+// length, 1e6: the 32-node example model 2.57 / 2.57 / 2.56, 20 nodes 2.17 / 2.17 / 2.18, 36 nodes 4.28 / 4.21 / 4.18
+// (3e4 and 1e3 of each: the same within 2 %).
 constexpr int MB_LOCK_STARTS = MB_LOCK_SMALL ? 8 : mbg_gate_rounds <= 2 ? 4 : 2;
 #ifndef MB_LOCK_BLOCKS
 #define MB_LOCK_BLOCKS 5
